@@ -567,17 +567,26 @@ __global__ void extract_keys_kernel(const unsigned long long* packed, uint64_t n
     }
 }
 
-// Output group i from its slot s ([key][count][value limbs...]).
-// (key: the slot's packed key word.)
+// The word of a group's slot that is not zero when the group has rows:
+// [key][count][...] hash slots, one-word slots and direct accumulators.
+__device__ __forceinline__ uint32_t count_word(const HashFormat& F) {
+    return (F.hpack || F.direct_acc) ? 0u : 1u;
+}
+
+// Output group i from its slot s ([key][count][value limbs...], or the direct
+// accumulators' [count lo][count hi][value limbs...]).
+// (key: the slot's packed key word, or its group index.)
 __device__ __forceinline__ void write_group(const unsigned long long* s, unsigned long long key, uint64_t i,
                                             const HashFormat& F, uint64_t* keys_out, tgp_agg_value* vals_out) {
     if (keys_out)
         for (uint32_t k = 0; k < F.nkey; ++k)
-            keys_out[i * F.nkey + k] = static_cast<uint64_t>(F.key_min[k]) + ((key >> F.key_shift[k]) & F.key_mask[k]);
+            keys_out[i * F.nkey + k] = static_cast<uint64_t>(F.key_min[k]) +
+                                       (F.direct_acc ? (key / F.key_div[k]) % F.key_mod[k]
+                                                     : (key >> F.key_shift[k]) & F.key_mask[k]);
     if (!vals_out) return;
     // One-word slots (F.hpack): the count above `hpack_shift`, below it the
     // sum of (value - bias) over the slot's rows.
-    const uint64_t cnt = F.hpack ? (F.hpack_shift < 64 ? s[0] >> F.hpack_shift : 0ull) : s[1];
+    const uint64_t cnt = F.hpack ? (F.hpack_shift < 64 ? s[0] >> F.hpack_shift : 0ull) : s[count_word(F)];
     for (uint32_t a = 0; a < F.nagg; ++a) {
         tgp_agg_value o;
         o.count = cnt;
@@ -619,8 +628,8 @@ __global__ void format_hash_groups_kernel(const unsigned long long* packed, cons
     }
 }
 
-// Directly indexed group tables (slot = key; a slot is occupied when its
-// count is not zero, its key word is never written): the occupied slots, in
+// Directly indexed group tables (slot = key or group index; a slot is occupied
+// when its count is not zero): the occupied slots, in
 // slot order, are the groups in ascending key order, so the result is written
 // straight from the table at positions from a prefix count of occupied
 // slots, with no gather and no sort. Block b covers slots
@@ -632,10 +641,9 @@ constexpr int kDirPerThread = 16;
 constexpr uint64_t kDirChunk = static_cast<uint64_t>(kAuxThreads) * kDirPerThread;
 
 __global__ void __launch_bounds__(kAuxThreads) count_direct_kernel(const unsigned long long* htab, uint64_t nslots,
-                                                                   uint32_t stride, unsigned long long* counts) {
+                                                                   uint32_t stride, uint32_t occ,
+                                                                   unsigned long long* counts) {
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kDirChunk;
-    // The count word: [key][count][...] slots, or the whole one-word slot.
-    const uint32_t occ = stride > 1 ? 1u : 0u;
     uint32_t c = 0;
 #pragma unroll 4
     for (int j = 0; j < kDirPerThread; ++j) {
@@ -661,10 +669,11 @@ __global__ void __launch_bounds__(kAuxThreads) format_direct_kernel(const unsign
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kDirChunk;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     unsigned long long run = offsets[blockIdx.x];
+    const uint32_t cw = count_word(F);
     for (int j = 0; j < kDirPerThread; ++j) {
         const uint64_t i = base + static_cast<uint64_t>(j) * kAuxThreads + threadIdx.x;
         const unsigned long long* s = htab + i * F.hstride;
-        const bool occ = i < nslots && s[F.hstride > 1 ? 1 : 0] != 0ull;
+        const bool occ = i < nslots && s[cw] != 0ull;
         const uint32_t mask = __ballot_sync(0xffffffffu, occ);
         if (lane == 0) wsum[warp] = __popc(mask);
         __syncthreads();
@@ -714,7 +723,7 @@ size_t direct_groups_scratch(uint64_t nslots) {
     return (nb + 1) * 16 + tmp + 256;
 }
 
-cudaError_t count_direct_groups(const unsigned long long* htab, uint64_t nslots, uint32_t stride, void* scratch,
+cudaError_t count_direct_groups(const unsigned long long* htab, uint64_t nslots, const HashFormat& F, void* scratch,
                                 size_t scratch_bytes, unsigned long long* total, cudaStream_t st) {
     const uint64_t nb = direct_groups_blocks(nslots);
     unsigned long long* counts = static_cast<unsigned long long*>(scratch);
@@ -724,7 +733,8 @@ cudaError_t count_direct_groups(const unsigned long long* htab, uint64_t nslots,
     // counts[nb] = 0, so offsets[nb] is the number of occupied slots.
     cudaError_t e = cudaMemsetAsync(counts + nb, 0, 8, st);
     if (e != cudaSuccess) return e;
-    if (nb) count_direct_kernel<<<static_cast<unsigned>(nb), kAuxThreads, 0, st>>>(htab, nslots, stride, counts);
+    if (nb) count_direct_kernel<<<static_cast<unsigned>(nb), kAuxThreads, 0, st>>>(
+            htab, nslots, F.hstride, (F.hpack || F.direct_acc) ? 0u : 1u, counts);
     e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, offsets, static_cast<int>(nb + 1), st);
     if (e != cudaSuccess) return e;
     return cudaMemcpyAsync(total, offsets + nb, 8, cudaMemcpyDeviceToDevice, st);

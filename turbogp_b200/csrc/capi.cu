@@ -23,6 +23,8 @@ namespace {
 constexpr unsigned long long kEmptySlot = ~0ull;
 constexpr uint64_t kDirectMaxGroups = 1ull << 22;
 constexpr uint64_t kHashDirectMax = 1ull << 27;   // key values of a directly indexed group table
+constexpr uint64_t kDeviceFormatGroups = 1024;         // direct groups formatted on the device from here on
+constexpr size_t kStagedResultBytes = 4u << 20;        // formatted results that come back through ctx->hpin
 constexpr size_t kJoinSmemCap = 144u << 10;        // shared memory per CTA of a payload-join scan (see size_smem)
 
 int fail(tgp_ctx* ctx, int st, const std::string& m) {
@@ -1969,10 +1971,17 @@ static void bound_presum(tgp_ctx* ctx, QueryState& qs) {
 // count in the top bits (enough for every row), the sum of (value - its
 // minimum) below. Groups formatted straight from the table only (no top-N,
 // at most kMaxFormatAggs aggregates).
+//
+// Direct accumulators in global memory (MODE_GROUP_GLOBAL, placed there by
+// the planner's rule) move to one-word slots on the same conditions: a slot
+// is 8 bytes instead of 32 or 48 and a row's global update one add instead
+// of two (40M rows, 500K Zipf(1.1) keys: accumulate, clear and read the
+// table 316 us -> see the streaming kernel's figures).
 static void plan_one_word_slots(QueryState& qs, const tgp_query* q, bool topn) {
     Plan& P = qs.b->P;
     const Builder& b = *qs.b;
-    if (!(qs.mode == MODE_GROUP_HASH && P.hdirect && P.hash_fast && P.nval <= 1 && !topn &&
+    const bool global = qs.mode == MODE_GROUP_GLOBAL && qs.kn.placement == 0;
+    if (!(((qs.mode == MODE_GROUP_HASH && P.hdirect) || global) && P.hash_fast && P.nval <= 1 && !topn &&
           q->nagg <= static_cast<uint32_t>(kMaxFormatAggs) && P.ngkey == 1 && P.gkey[0].shift == 0 &&
           (!P.hsm_slots || P.hsm_key32) && (P.nval == 0 || !b.val_big[0])))
         return;
@@ -1987,6 +1996,13 @@ static void plan_one_word_slots(QueryState& qs, const tgp_query* q, bool topn) {
         P.hpack_shift = shift;
         P.hpack_bias = P.nval ? static_cast<int64_t>(b.val_lo[0]) : 0;
         P.hstride = 1;
+        if (global) {
+            qs.mode = MODE_GROUP_HASH;
+            qs.hcap = std::max<uint64_t>(16, qs.ngroups_direct);
+            P.hdirect = 1;
+            P.hlog2 = log2u(next_pow2(qs.hcap));
+            P.hmask = qs.hcap - 1;
+        }
     }
 }
 
@@ -2066,6 +2082,16 @@ static void host_topn(const TopNReq& tn, uint32_t nkey, uint32_t nagg, const std
     result->ngroups = m;
 }
 
+// Whether a run of the query formats its groups on the device straight from
+// their table: directly indexed slots, and direct accumulators of many groups
+// (few are decoded on the host from the one readback that carries the
+// counters, without the extra kernels and the second wait).
+static bool formats_direct(const QueryState& qs, const tgp_query* q) {
+    if (q->nagg > static_cast<uint32_t>(kMaxFormatAggs)) return false;
+    if (qs.mode == MODE_GROUP_HASH) return qs.b->P.hdirect != 0;
+    return q->ngroup != 0 && qs.ngroups_direct >= kDeviceFormatGroups;
+}
+
 static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tgp_agg_value* vals_out,
                         uint64_t group_cap, tgp_query_result* result, const TopNReq* tn) {
     if (!ctx || !q || !result) return fail(ctx, TGP_INVALID_ARG, "null argument");
@@ -2073,6 +2099,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     if (tn && tn->agg >= q->nagg) return fail(ctx, TGP_INVALID_ARG, "ORDER BY aggregate index out of range");
     QueryState qs;
     TGP_TRY(plan_query(ctx, q, qs, scan_kernel_static_smem()));
+    plan_one_word_slots(qs, q, tn != nullptr);
     Builder& b = *qs.b;
     Plan& P = b.P;
     const Table* T = qs.T;
@@ -2087,15 +2114,16 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     const std::vector<AggMap>& amap = qs.amap;
     const unsigned __int128 D = qs.D;
     const uint32_t total_bits = qs.total_bits;
-    (void)nv1;
 
-    plan_one_word_slots(qs, q, tn != nullptr);
-
-    // Scratch: accumulators (direct/scalar) or hash table, counters, error word.
+    // Scratch: accumulators (direct/scalar) or hash table, counters, error
+    // word, and the prefix counts of results formatted on the device.
     const uint64_t acc_words = qs.acc_words();
     const uint64_t htab_words = hcap * P.hstride;
+    const bool device_fmt = !tn && formats_direct(qs, q);
+    const uint64_t fmt_slots = mode == MODE_GROUP_HASH ? hcap : ngroups_direct;
+    const size_t fmt_scratch = device_fmt ? direct_groups_scratch(fmt_slots) : 0;
     Carve cv;
-    TGP_TRY(arena_reserve(ctx, acc_words * 8 + htab_words * 8 + 1024, &cv));
+    TGP_TRY(arena_reserve(ctx, acc_words * 8 + htab_words * 8 + fmt_scratch + 2048, &cv));
     // One result block [counters: 4 words][error word: 2 words][accumulators],
     // cleared with one memset and read back with one copy.
     const uint64_t block_words = qs.block_words();
@@ -2104,13 +2132,17 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     P.err = reinterpret_cast<uint32_t*>(block + 4);
     P.acc = acc_words ? block + 6 : cv.take<unsigned long long>(2);
     P.htab = mode == MODE_GROUP_HASH ? cv.take<unsigned long long>(htab_words) : nullptr;
-    bool has_minmax = false;
-    for (uint32_t v = 0; v < P.nval; ++v) has_minmax |= (P.val[v].kind == VK_MIN || P.val[v].kind == VK_MAX);
-    if (acc_words && has_minmax) {
+    uint8_t* fmt = device_fmt ? cv.take<uint8_t>(fmt_scratch) : nullptr;
+    if (acc_words && qs.has_minmax()) {
+        // Every group's accumulators from one image, written on the device.
         TGP_CUDA(cudaMemsetAsync(block, 0, 48, ctx->stream));
-        std::vector<unsigned long long> img;
-        init_acc_image(P, ngroups_direct, &img);
-        TGP_TRY(upload(ctx, P.acc, img.data(), img.size() * 8));
+        std::vector<unsigned long long> one;
+        init_acc_image(P, 1, &one);
+        SlotImage img;
+        std::memset(&img, 0, sizeof(img));
+        img.stride = nv1 * 2;
+        std::copy(one.begin(), one.end(), img.w);
+        TGP_CUDA(launch_fill_slots(P.acc, ngroups_direct, img, ctx->sms, ctx->stream));
     } else {
         TGP_CUDA(cudaMemsetAsync(block, 0, block_words * 8, ctx->stream));
     }
@@ -2139,29 +2171,8 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         if (!done) TGP_TRY(launch(ctx, P, mode, acc128));
     }
 
-    TGP_TRY(pinned_reserve(ctx, block_words * 8));
-    TGP_CUDA(cudaMemcpyAsync(ctx->hpin, block, block_words * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
-    const unsigned long long* hb = reinterpret_cast<const unsigned long long*>(ctx->hpin);
-    unsigned long long counters[4] = {hb[0], hb[1], hb[2], hb[3]};
-    const uint32_t err = static_cast<uint32_t>(hb[4] & 0xffffffffull);
-    TGP_TRY(check_kernel_err(ctx, err));
-
-    result->rows_scanned = T->rows;
-    result->rows_selected = counters[0];
-    result->flags = (err & kErrRowOverflow) ? TGP_RESULT_ROW_OVERFLOW : 0u;
     const uint32_t nagg = q->nagg;
-
-    if (mode != MODE_GROUP_HASH) {
-        if (!tn) return decode_direct(ctx, qs, hb, keys_out, vals_out, group_cap, result);
-        std::vector<uint64_t> ak(std::max<uint64_t>(1, ngroups_direct * q->ngroup));
-        std::vector<tgp_agg_value> av(std::max<uint64_t>(1, ngroups_direct * q->nagg));
-        TGP_TRY(decode_direct(ctx, qs, hb, ak.data(), av.data(), ngroups_direct, result));
-        host_topn(*tn, q->ngroup, q->nagg, ak, av, result->ngroups, amap[tn->agg].func, keys_out, vals_out, result);
-        return TGP_OK;
-    }
-
-    auto hash_format = [&]() {
+    auto group_format = [&]() {
         HashFormat F;
         std::memset(&F, 0, sizeof(F));
         F.nkey = q->ngroup;
@@ -2171,10 +2182,16 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         F.hpack = P.hpack;
         F.hpack_shift = P.hpack_shift;
         F.hpack_bias = P.hpack_bias;
+        if (mode != MODE_GROUP_HASH) {
+            F.hstride = nv1 * 2;
+            F.direct_acc = 1;
+        }
         for (uint32_t k = 0; k < q->ngroup; ++k) {
             F.key_shift[k] = P.gkey[k].shift;
             F.key_mask[k] = bits[k] >= 64 ? ~0ull : ((1ull << bits[k]) - 1);
             F.key_min[k] = kmin[k];
+            F.key_div[k] = F.direct_acc ? P.gkey[k].stride : 1;
+            F.key_mod[k] = F.direct_acc ? qs.dom[k] : 1;
         }
         for (uint32_t a = 0; a < nagg; ++a) {
             F.func[a] = static_cast<uint8_t>(amap[a].func);
@@ -2183,49 +2200,73 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         }
         return F;
     };
+    // Groups in index (= key) order straight from the table: the number of
+    // occupied slots comes back with the counters (word 2), so one wait covers
+    // the scan and the count.
+    const unsigned long long* table = mode == MODE_GROUP_HASH ? P.htab : P.acc;
+    uint64_t back_words = block_words;
+    if (device_fmt) {
+        back_words = 6;
+        TGP_CUDA(count_direct_groups(table, fmt_slots, group_format(), fmt, fmt_scratch, P.counters + 2, ctx->stream));
+    }
+
+    TGP_TRY(pinned_reserve(ctx, back_words * 8));
+    TGP_CUDA(cudaMemcpyAsync(ctx->hpin, block, back_words * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
+    const unsigned long long* hb = reinterpret_cast<const unsigned long long*>(ctx->hpin);
+    unsigned long long counters[4] = {hb[0], hb[1], hb[2], hb[3]};
+    const uint32_t err = static_cast<uint32_t>(hb[4] & 0xffffffffull);
+    TGP_TRY(check_kernel_err(ctx, err));
+
+    result->rows_scanned = T->rows;
+    result->rows_selected = counters[0];
+    result->flags = (err & kErrRowOverflow) ? TGP_RESULT_ROW_OVERFLOW : 0u;
+
+    if (device_fmt) {
+        const uint64_t ng = counters[2];
+        result->ngroups = ng;
+        if (ng > group_cap) return fail(ctx, TGP_CAPACITY, "group buffer too small");
+        const HashFormat F = group_format();
+        const size_t kbytes = (keys_out ? ng * q->ngroup * 8 : 0), vbytes = (vals_out ? ng * nagg * sizeof(tgp_agg_value) : 0);
+        const size_t vofs = (kbytes + 255) & ~size_t{255};
+        uint8_t* buf = nullptr;
+        TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&buf), vofs + vbytes, "group format allocation failed"));
+        cudaError_t e = format_direct_groups(table, fmt_slots, fmt, ng, F, kbytes ? reinterpret_cast<uint64_t*>(buf) : nullptr,
+                                             vbytes ? reinterpret_cast<tgp_agg_value*>(buf + vofs) : nullptr, ctx->stream);
+        // Small results come back in one copy to page-locked staging.
+        const bool staged = vofs + vbytes <= kStagedResultBytes;
+        if (staged && e == cudaSuccess && (kbytes || vbytes)) {
+            if (int st = pinned_reserve(ctx, vofs + vbytes)) {
+                dev_free(ctx, buf);
+                return st;
+            }
+            e = cudaMemcpyAsync(ctx->hpin, buf, vofs + vbytes, cudaMemcpyDeviceToHost, ctx->stream);
+        } else {
+            if (e == cudaSuccess && kbytes) e = cudaMemcpyAsync(keys_out, buf, kbytes, cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess && vbytes)
+                e = cudaMemcpyAsync(vals_out, buf + vofs, vbytes, cudaMemcpyDeviceToHost, ctx->stream);
+        }
+        dev_free(ctx, buf);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("group format: ") + cudaGetErrorString(e));
+        if (staged) {
+            if (kbytes) std::memcpy(keys_out, ctx->hpin, kbytes);
+            if (vbytes) std::memcpy(vals_out, ctx->hpin + vofs, vbytes);
+        }
+        return TGP_OK;
+    }
+    if (mode != MODE_GROUP_HASH) {
+        if (!tn) return decode_direct(ctx, qs, hb, keys_out, vals_out, group_cap, result);
+        std::vector<uint64_t> ak(std::max<uint64_t>(1, ngroups_direct * q->ngroup));
+        std::vector<tgp_agg_value> av(std::max<uint64_t>(1, ngroups_direct * q->nagg));
+        TGP_TRY(decode_direct(ctx, qs, hb, ak.data(), av.data(), ngroups_direct, result));
+        host_topn(*tn, q->ngroup, q->nagg, ak, av, result->ngroups, amap[tn->agg].func, keys_out, vals_out, result);
+        return TGP_OK;
+    }
+
     // Hash groups: gather occupied slots, sort by key on the host.
     // Counter word 2 counts the gathered slots.
     TGP_CUDA(cudaMemsetAsync(P.counters + 2, 0, 8, ctx->stream));
-    if (P.hdirect && !tn && nagg <= static_cast<uint32_t>(kMaxFormatAggs)) {
-        // A directly indexed table holds the groups in key order already:
-        // count the occupied slots, then format them in place of a gather
-        // and a sort.
-        const size_t sb = direct_groups_scratch(hcap);
-        uint8_t* scr = nullptr;
-        TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&scr), sb, "group count allocation failed"));
-        unsigned long long ng = 0;
-        cudaError_t e = count_direct_groups(P.htab, hcap, P.hstride, scr, sb, P.counters + 2, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&ng, P.counters + 2, 8, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) {
-            dev_free(ctx, scr);
-            return fail(ctx, TGP_DEVICE_ERROR, std::string("group count: ") + cudaGetErrorString(e));
-        }
-        result->ngroups = ng;
-        if (ng > group_cap) {
-            dev_free(ctx, scr);
-            return fail(ctx, TGP_CAPACITY, "group buffer too small");
-        }
-        const HashFormat F = hash_format();
-        const size_t kbytes = (keys_out ? ng * q->ngroup * 8 : 0), vbytes = (vals_out ? ng * nagg * sizeof(tgp_agg_value) : 0);
-        uint8_t* buf = nullptr;
-        const size_t vofs = (kbytes + 255) & ~size_t{255};
-        if (int st = dev_alloc(ctx, reinterpret_cast<void**>(&buf), std::max<size_t>(vofs + vbytes, 256),
-                               "group format allocation failed")) {
-            dev_free(ctx, scr);
-            return st;
-        }
-        uint64_t* dkeys = kbytes ? reinterpret_cast<uint64_t*>(buf) : nullptr;
-        tgp_agg_value* dvals = vbytes ? reinterpret_cast<tgp_agg_value*>(buf + vofs) : nullptr;
-        e = format_direct_groups(P.htab, hcap, scr, ng, F, dkeys, dvals, ctx->stream);
-        if (e == cudaSuccess && kbytes) e = cudaMemcpyAsync(keys_out, dkeys, kbytes, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess && vbytes) e = cudaMemcpyAsync(vals_out, dvals, vbytes, cudaMemcpyDeviceToHost, ctx->stream);
-        dev_free(ctx, buf);
-        dev_free(ctx, scr);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("group format: ") + cudaGetErrorString(e));
-        return TGP_OK;
-    }
     unsigned long long* packed = nullptr;
     const uint64_t max_groups = std::min<uint64_t>(hcap, static_cast<uint64_t>(std::min<unsigned __int128>(D, hcap)));
     TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&packed), std::max<uint64_t>(max_groups, 1) * P.hstride * 8,
@@ -2243,7 +2284,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     if (nagg <= static_cast<uint32_t>(kMaxFormatAggs)) {
         // Sort by packed key (= ascending lexicographic key order, key 0 in
         // the top bits) and format on the device; copy the caller's arrays once.
-        const HashFormat F = hash_format();
+        const HashFormat F = group_format();
         // Top-N: only the first min(limit, ng) groups in the aggregate's order
         // are formatted and copied.
         const uint64_t nout = tn ? std::min<uint64_t>(tn->limit, ng) : ng;
@@ -2340,13 +2381,16 @@ int tgp_query_footprint(tgp_ctx* ctx, const tgp_query* q, uint64_t* device_bytes
         const uint64_t max_groups =
             std::min<uint64_t>(qs.hcap, static_cast<uint64_t>(std::min<unsigned __int128>(qs.D, qs.hcap)));
         bytes += qs.hcap * slot_bytes;                                    // the group table
-        if (P.hdirect && q->nagg <= static_cast<uint32_t>(kMaxFormatAggs)) {
+        if (formats_direct(qs, q)) {
             bytes += direct_groups_scratch(qs.hcap);                      // prefix counts of occupied slots
         } else {
             bytes += max_groups * slot_bytes;                             // gathered occupied slots
             bytes += format_hash_groups_scratch(max_groups, qs.total_bits);  // device sort
         }
         bytes += max_groups * (8ull * q->ngroup + sizeof(tgp_agg_value) * q->nagg) + 512;  // formatted result
+    } else if (formats_direct(qs, q)) {
+        bytes += direct_groups_scratch(qs.ngroups_direct) +
+                 qs.ngroups_direct * (8ull * q->ngroup + sizeof(tgp_agg_value) * q->nagg) + 512;
     }
     *device_bytes = bytes;
     return TGP_OK;

@@ -350,6 +350,12 @@ struct HashFormat {
     uint32_t nkey, nagg, hstride, sum64;  // sum64: value limbs hold int64 sums (hi = sign of lo)
     uint32_t hpack, hpack_shift;          // one-word direct slots (Plan::hpack)
     int64_t hpack_bias;
+    // Direct-indexed accumulators ([count lo][count hi][v0 lo][v0 hi]...,
+    // hstride words per group): key k of group index g is
+    // key_min + (g / key_div) % key_mod. 0 = hash-table slots.
+    uint32_t direct_acc;
+    uint32_t _pad;
+    uint64_t key_div[kMaxGroupKeys], key_mod[kMaxGroupKeys];
     uint32_t key_shift[kMaxGroupKeys];
     uint64_t key_mask[kMaxGroupKeys];
     int64_t key_min[kMaxGroupKeys];
