@@ -62,3 +62,32 @@ def test_many_direct_groups_of_several_keys(ctx, n):
         for where in (None, q < 20):
             same(t.aggregate(aggs, keys, where, group_cap=1), oracle.aggregate(h, CT, aggs, keys, where))
     t.drop()
+
+
+@pytest.mark.parametrize("n,groups", [(1, 1), (2_047, 300), (2_048, 1_200), (150_001, 2_500), (150_001, 9_001)])
+def test_limb_tables_of_sums_and_extremes(ctx, n, groups):
+    """One shared table word per extreme and per small sum, two per wide sum:
+    negative values, ranges of and past 2^32, joins through a payload, the
+    same query forced onto the other placements and captured."""
+    h = keyed(n, groups, -17, np.int32, 11 + n)
+    h["edge"] = np.where(np.arange(n) % 2 == 0, -2**31, 2**31 - 1).astype(np.int64)   # a range of 2^32 - 1
+    t = ctx.register(h)
+    v, u, w = col("v"), col("u"), col("w")
+    shapes = [[count_star(), min_(v), max_(v)], [min_(100 - v), max_(v * u), sum_(u), count_col(v)],
+              [sum_(w), min_(col("edge")), max_(col("edge"))], [min_(w), sum_(v)], [avg(v * u), max_(u), sum_(w * 2)]]
+    try:
+        for placement in (0, 4, 2, 3):
+            ctx.set_default_variant(placement=placement)
+            for aggs in shapes:
+                for where in (None, (u >= 30) & (v < 500), v > 5_000):
+                    same(t.aggregate(aggs, ("key",), where), oracle.aggregate(h, None, aggs, ("key",), where))
+    finally:
+        ctx.set_default_variant(placement=0)
+    pq = t.prepare(shapes[1], ("key",), u < 200, group_cap=16_384)
+    if groups < 9_000:
+        pq.capture()
+    same(pq.run(), oracle.aggregate(h, None, shapes[1], ("key",), u < 200))
+    pq.drop_graph()
+    same(ctx.submit([pq, t.prepare(shapes[4], ("key",), None, group_cap=16_384)]).wait()[1],
+         oracle.aggregate(h, None, shapes[4], ("key",), None))
+    t.drop()

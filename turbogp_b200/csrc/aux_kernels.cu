@@ -637,7 +637,7 @@ __global__ void format_hash_groups_kernel(const unsigned long long* packed, cons
 // slots, a device scan makes them offsets, pass 2 writes each block's groups
 // in order (slot base + j * kAuxThreads + thread, j ascending, so a warp's
 // ballot and the block's warp totals give each slot's rank).
-constexpr int kDirPerThread = 16;
+constexpr int kDirPerThread = 1;
 constexpr uint64_t kDirChunk = static_cast<uint64_t>(kAuxThreads) * kDirPerThread;
 
 __global__ void __launch_bounds__(kAuxThreads) count_direct_kernel(const unsigned long long* htab, uint64_t nslots,

@@ -23,7 +23,7 @@ namespace {
 constexpr unsigned long long kEmptySlot = ~0ull;
 constexpr uint64_t kDirectMaxGroups = 1ull << 22;
 constexpr uint64_t kHashDirectMax = 1ull << 27;   // key values of a directly indexed group table
-constexpr uint64_t kDeviceFormatGroups = 1024;         // direct groups formatted on the device from here on
+constexpr uint64_t kDeviceFormatGroups = 4096;         // direct groups formatted on the device from here on
 constexpr size_t kStagedResultBytes = 4u << 20;        // formatted results that come back through ctx->hpin
 constexpr size_t kJoinSmemCap = 144u << 10;        // shared memory per CTA of a payload-join scan (see size_smem)
 
@@ -1584,6 +1584,37 @@ struct BucketSpec {
     uint32_t nbuckets[kMaxGroupKeys];
 };
 
+// Lays out one group's words of the 32-bit limb tables (Plan::s32_*): the row
+// count, then per value two limbs of a sum, one word of a sum whose partial
+// in a CTA's table provably fits 32 bits, or one word of an extreme whose
+// value range is below 2^32. Returns the words per group, 0 when a value
+// has no such form. Fixed-shape value programs keep two words per value.
+static uint32_t plan_s32_words(Builder& b, uint64_t rows, uint32_t sms, bool fixed_values) {
+    Plan& P = b.P;
+    // A CTA's tiles at any grid launch() takes (at least one CTA per SM, or
+    // one per tile): its tables' rows.
+    const uint64_t ntiles = (rows + kTileRows - 1) / kTileRows;
+    const uint64_t ctas = std::max<uint64_t>(1, std::min<uint64_t>(ntiles, sms));
+    const unsigned __int128 rows_cta = static_cast<unsigned __int128>((ntiles + ctas - 1) / ctas) * kTileRows;
+    uint32_t w = 1;
+    for (uint32_t v = 0; v < P.nval; ++v) {
+        const uint8_t kind = P.val[v].kind;
+        P.s32_off[v] = static_cast<uint8_t>(w);
+        if (kind == VK_MIN || kind == VK_MAX) {
+            if (b.val_big[v] || b.val_hi[v] - b.val_lo[v] > 0xffffffffll) return 0;
+            P.s32_kind[v] = kind == VK_MIN ? S32_MIN : S32_MAX;
+            P.s32_ref[v] = static_cast<int64_t>(kind == VK_MIN ? b.val_hi[v] : b.val_lo[v]);
+            w += 1;
+            continue;
+        }
+        const unsigned __int128 most = static_cast<unsigned __int128>(std::max(abs128(b.val_lo[v]), abs128(b.val_hi[v])));
+        const bool narrow = !b.val_big[v] && !fixed_values && rows_cta * most < (static_cast<unsigned __int128>(1) << 31);
+        P.s32_kind[v] = narrow ? S32_NARROW : S32_WIDE;
+        w += narrow ? 1 : 2;
+    }
+    return w;
+}
+
 static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t static_smem,
                       const std::vector<uint32_t>* preseed = nullptr, bool dry = false,
                       const BucketSpec* bucket = nullptr) {
@@ -1740,12 +1771,11 @@ static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t s
             const size_t s256 = budget > private_bytes(256) ? (budget - private_bytes(256)) / st : 0;
             if (s512 == 2 && std::min<size_t>(s256, static_cast<size_t>(kn.max_stages)) >= 4) nt = 256;
         }
-        // Per-warp shared tables of 32-bit limbs with native shared atomics
-        // (SUM / COUNT(col) values only): exact when every table's sums stay
-        // below 2^63 in magnitude, which rows x max|value| < 2^63 proves (at
-        // most one build match per probe row). Taken when the private
-        // accumulators do not fit (or a variant asks for it).
-        const uint32_t s32_words = 1 + 2 * P.nval;
+        // Per-warp shared tables of 32-bit words with native shared atomics:
+        // exact when every table's sums stay below 2^63 in magnitude, which
+        // rows x max|value| < 2^63 proves (at most one build match per probe
+        // row), and every extreme's value range is below 2^32. Taken when
+        // the private accumulators do not fit (or a variant asks for it).
         const uint32_t s32_nt = kn.threads == 256 ? 256u : 512u;
         // Bucketed (merged) plans take the limb tables whenever they are
         // exact: the private placement has no dense path for bucket keys
@@ -1754,14 +1784,16 @@ static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t s
         // the fixed shapes: the 60M x 1.5M join probe ran 0.332 ms on the
         // limb tables (512 threads, four stages) against 0.374-0.387 ms with
         // private accumulators (autotuner, gated CUDA events).
-        bool join_s32 = false;
-        if (J && pay_ok && kn.placement == 0 && kn.dense && kn.shapes && !P.check_ovf &&
+        bool fixed_values = false;   // the value program is one of the fixed shapes
+        if ((J || bucket || kn.placement == 4 || nt == 0) && (!J || pay_ok) && kn.dense && kn.shapes && !P.check_ovf &&
             compile_chain(b, pay_ok, static_cast<uint32_t>(kMaxGroupKeys))) {
             const uint32_t dv = P.dense_vec;
             P.dense_vec = 1;
-            join_s32 = value_shape_of(P) != 0;
+            fixed_values = value_shape_of(P) != 0;
             P.dense_vec = dv;
         }
+        const bool join_s32 = J && kn.placement == 0 && fixed_values;
+        const uint32_t s32_words = plan_s32_words(b, T->rows, static_cast<uint32_t>(ctx->sms), fixed_values);
         const bool prefer_s32 = kn.placement == 4 || (bucket != nullptr && kn.placement == 0) || join_s32;
         auto s32_bytes = [&](uint32_t copies) -> size_t {
             return static_cast<size_t>(copies) * ngroups_direct * s32_words * 4;
@@ -1770,11 +1802,9 @@ static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t s
         {
             bool ok = !b.unbounded && (!J || J->unique) && kn.placement != 2 && kn.placement != 3 &&
                       (nt == 0 || prefer_s32);
-            for (uint32_t v = 0; ok && v < P.nval; ++v)
-                ok = P.val[v].kind == VK_SUM || P.val[v].kind == VK_COUNT_NZ;
             const unsigned __int128 bound = static_cast<unsigned __int128>(std::max<uint64_t>(T->rows, 1)) *
                                             std::max<uint64_t>(b.max_abs_val, 1);
-            ok = ok && bound < (static_cast<unsigned __int128>(1) << 63);
+            ok = ok && s32_words && bound < (static_cast<unsigned __int128>(1) << 63);
             if (ok) {
                 const size_t st = P.stage_bytes;
                 uint32_t copies = s32_nt / 32;

@@ -62,6 +62,20 @@ __device__ __forceinline__ void sts_u64(uint32_t a, unsigned long long v) {
     asm volatile("st.shared.u64 [%0+%1], %2;" ::"r"(a), "n"(OFF), "l"(v) : "memory");
 }
 
+// Native 32-bit shared atomics on shared addresses (the red forms return
+// nothing, so a thread does not wait for them).
+__device__ __forceinline__ uint32_t atom_add_shared(uint32_t a, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ void red_add_shared(uint32_t a, uint32_t v) {
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void red_max_shared(uint32_t a, uint32_t v) {
+    asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
                  : "memory");

@@ -92,6 +92,14 @@ constexpr uint32_t kShapeScalar = 0xffffu;
 // Postfix program opcodes: values < kMaxLeaves push leaf i.
 enum : uint8_t { OP_AND = 0x80, OP_OR = 0x81, OP_NOT = 0x82 };
 
+// Value words of the 32-bit limb tables. Every word starts at 0.
+enum : uint8_t {
+    S32_WIDE = 0,    // a SUM as [lo u32, hi i32]: a returning add and the carry
+    S32_NARROW = 1,  // a SUM whose table partial fits i32 (host-proven): one non-returning add
+    S32_MIN = 2,     // the largest (range end - value), u32: a maximum, 0 = nothing below the end
+    S32_MAX = 3      // the largest (value - range start), u32
+};
+
 // Value accumulator kinds.
 enum : uint8_t { VK_SUM = 0, VK_MIN = 1, VK_MAX = 2, VK_COUNT_NZ = 3 };
 
@@ -248,11 +256,14 @@ struct alignas(16) Plan {
                                     // of one staged factor each (at most two): the column path
     uint32_t group_fast;            // batch launches: every plan of this plan's morsel group is a scalar
                                     // fast-path plan with the same register leaf columns and values
-    // MODE_GROUP_SHARED32: tables of s32_words u32 words per group ([count]
-    // [lo, hi] per value), one per s32_copies groups of warps (warp w uses
-    // table w % s32_copies).
+    // MODE_GROUP_SHARED32: tables of s32_words u32 words per group ([count],
+    // then value v's words from s32_off[v] as s32_kind[v] says), one per
+    // s32_copies groups of warps (warp w uses table w % s32_copies).
     uint32_t s32_copies;
     uint32_t s32_words;
+    uint8_t s32_off[kMaxVals];
+    uint8_t s32_kind[kMaxVals];   // S32_*
+    int64_t s32_ref[kMaxVals];    // S32_MIN: the value range's upper end, S32_MAX: its lower end
     // Failure-path test hook (tgp_debug_fail_next_scan): tile + 1 whose stage
     // copy the producer skips (0 = none), and the bounded waits' limit in ns
     // (0 = kWaitLimitNs).

@@ -593,6 +593,26 @@ __device__ __forceinline__ bool presum_add(const Plan& P, uint8_t* extra, uint64
     return done;
 }
 
+// Adds value argument x to its words `e` of a 32-bit limb table with native
+// 32-bit shared atomics. The host proved every wide sum stays below 2^63 in
+// magnitude and every narrow one below 2^31, so the words recombine exactly.
+// Extremes are held as distances from the far end of the value's range, so
+// both are maxima over words that start at 0; a row that does not raise the
+// word (almost every one, once a group has seen a few rows) is one plain load.
+__device__ __forceinline__ void s32_add(uint32_t* e, uint32_t s32_kind, int64_t ref, int64_t x) {
+    if (s32_kind == S32_WIDE) {
+        const uint32_t xl = static_cast<uint32_t>(x);
+        const uint32_t old = atomicAdd(e, xl);
+        const int32_t add = static_cast<int32_t>(x >> 32) + ((old + xl < old) ? 1 : 0);
+        if (add) atomicAdd(reinterpret_cast<int*>(e + 1), add);
+    } else if (s32_kind == S32_NARROW) {
+        atomicAdd(e, static_cast<uint32_t>(x));
+    } else {
+        const uint32_t k = static_cast<uint32_t>(s32_kind == S32_MIN ? ref - x : x - ref);
+        if (k > *reinterpret_cast<volatile uint32_t*>(e)) atomicMax(e, k);
+    }
+}
+
 template <uint32_t MODE, bool ACC128, int NT>
 struct Sink {
     uint32_t ovf;
@@ -735,11 +755,7 @@ struct Sink {
                 }
             }
         } else if (MODE == MODE_GROUP_SHARED32) {
-            // Native 32-bit shared atomics on this warp group's table: the row
-            // count, and per value the low 32 bits (the returned old value
-            // gives the carry) and the signed high 32 bits. The host proved
-            // every table's sums stay below 2^63 in magnitude, so the limbs
-            // recombine exactly.
+            // This warp group's table: the row count and the values' words.
             const uint32_t g = group_index<TAIL>(P, stage, r0, rl, brow, gpay);
             uint32_t* tab = reinterpret_cast<uint32_t*>(extra) +
                             (static_cast<size_t>((t >> 5) & (P.s32_copies - 1u)) * P.ngroups + g) * P.s32_words;
@@ -749,10 +765,7 @@ struct Sink {
                 const ValDesc& V = P.val[v];
                 int64_t x = eval_val<TAIL>(P, V, stage, r0, rl, brow, ovf);
                 if (V.kind == VK_COUNT_NZ) x = x != 0 ? 1 : 0;
-                const uint32_t xl = static_cast<uint32_t>(x);
-                const uint32_t old = atomicAdd(&tab[1 + 2 * v], xl);
-                const int32_t add = static_cast<int32_t>(x >> 32) + ((old + xl < old) ? 1 : 0);
-                if (add) atomicAdd(reinterpret_cast<int*>(&tab[2 + 2 * v]), add);
+                s32_add(&tab[P.s32_off[v]], P.s32_kind[v], P.s32_ref[v], x);
             }
         } else if (MODE == MODE_GROUP_GLOBAL) {
             const uint32_t g = group_index<TAIL>(P, stage, r0, rl, brow, gpay);
@@ -852,17 +865,35 @@ struct Sink {
             const uint32_t W = P.s32_words, G = P.ngroups;
             for (uint32_t idx = t; idx < G * nv1; idx += NT) {
                 const uint32_t g = idx / nv1, v = idx % nv1;
-                // Sum the copies' limbs: counts as u64; a value as the exact
-                // int64 (hi << 32) + lo of each copy.
+                const uint32_t sk = v == 0 ? static_cast<uint32_t>(S32_WIDE) : P.s32_kind[v - 1];
+                // Sum the copies' limbs: counts as u64; a wide value as the
+                // exact int64 (hi << 32) + lo of each copy; extremes as the
+                // maximum over the copies, of a group with rows.
                 int64_t sum = 0;
+                uint32_t far = 0, rows = 0;
                 for (uint32_t c = 0; c < P.s32_copies; ++c) {
                     const uint32_t* e = tab + (static_cast<size_t>(c) * G + g) * W;
                     if (v == 0) {
                         sum += static_cast<int64_t>(e[0]);
-                    } else {
-                        const uint64_t hi = static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(e[2 * v])));
-                        sum = static_cast<int64_t>(static_cast<uint64_t>(sum) + ((hi << 32) | e[2 * v - 1]));
+                        continue;
                     }
+                    rows |= e[0];
+                    e += P.s32_off[v - 1];
+                    if (sk == S32_WIDE) {
+                        const uint64_t hi = static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(e[1])));
+                        sum = static_cast<int64_t>(static_cast<uint64_t>(sum) + ((hi << 32) | e[0]));
+                    } else if (sk == S32_NARROW) {
+                        sum += static_cast<int64_t>(static_cast<int32_t>(e[0]));
+                    } else {
+                        far = max(far, e[0]);
+                    }
+                }
+                if (sk == S32_MIN || sk == S32_MAX) {
+                    if (rows == 0) continue;
+                    const int64_t x = sk == S32_MIN ? P.s32_ref[v - 1] - static_cast<int64_t>(far)
+                                                    : P.s32_ref[v - 1] + static_cast<int64_t>(far);
+                    acc_global_i64(P.acc + 2ull * idx, sk == S32_MIN ? VK_MIN : VK_MAX, x);
+                    continue;
                 }
                 if (sum == 0) continue;
                 I128 a;
@@ -1170,8 +1201,7 @@ __device__ __forceinline__ void chain_private_tile(const Plan& P, uint8_t* extra
 // bucket tables, the join payload's build-side part) and the value program's
 // steps are computed for the thread's R rows column by column, then the
 // selected rows add to this warp group's table with native 32-bit shared
-// atomics: the row count, and per value the low limb (its returned old value
-// gives the carry) and the signed high limb.
+// atomics: the row count, and the words of each value (s32_add).
 // ---------------------------------------------------------------------------
 template <int NT>
 __device__ __forceinline__ void chain_s32_tile(const Plan& P, uint8_t* extra, const uint8_t* stage, uint32_t t,
@@ -1195,57 +1225,89 @@ __device__ __forceinline__ void chain_s32_tile(const Plan& P, uint8_t* extra, co
             for (int r = 0; r < R; ++r) g[r] += (x[r] - mn) * st;
         }
     }
-    const uint32_t W = P.s32_words;
-    // (s32_copies is a power of two.)
-    uint32_t* tab = reinterpret_cast<uint32_t*>(extra) + static_cast<size_t>((t >> 5) & (P.s32_copies - 1u)) * P.ngroups * W;
+    // Byte address of each row's words in this warp group's table (s32_copies
+    // is a power of two).
+    const uint32_t W4 = P.s32_words * 4u;
+    const uint32_t tab = smem_addr(extra) + ((t >> 5) & (P.s32_copies - 1u)) * P.ngroups * W4;
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-        if ((m >> r) & 1u) atomicAdd(&tab[g[r] * W], 1u);
+    for (int r = 0; r < R; ++r) {
+        g[r] = tab + g[r] * W4;
+        if ((m >> r) & 1u) red_add_shared(g[r], 1u);
+    }
+    // The steps run on 64-bit products, except a first factor in 32-bit
+    // arithmetic that goes to one-word slots only through its low word.
     int64_t cur[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) cur[r] = 0;
 #pragma unroll 1
     for (uint32_t s = 0; s < P.chain.nsteps; ++s) {
         const ChainStep& S = P.chain.s[s];
-        int64_t f[R];
-        if (S.flags & CS_COL) {
-            if (S.flags & CS_NARROW) {
+        const uint32_t fl = S.flags;
+        if (fl & CS_COL) {
+            if (fl & CS_NARROW) {
                 uint32_t x[R];
                 load_cells32<R>(stage + S.soff, S.dtype, t, x);
+                const uint32_t mu = static_cast<uint32_t>(S.mul32), ad = static_cast<uint32_t>(S.add32);
+                if (fl & CS_CHAIN) {
 #pragma unroll
-                for (int r = 0; r < R; ++r)
-                    f[r] = static_cast<int32_t>(static_cast<uint32_t>(S.mul32) * x[r] + static_cast<uint32_t>(S.add32));
+                    for (int r = 0; r < R; ++r)
+                        cur[r] = static_cast<int64_t>(static_cast<uint64_t>(cur[r]) *
+                                                      static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(mu * x[r] + ad))));
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) cur[r] = static_cast<int32_t>(mu * x[r] + ad);
+                }
             } else {
                 int64_t x[R];
                 load_cells64<R>(stage + S.soff, S.dtype, t, x);
+                if (!(fl & CS_IDENT)) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        x[r] = static_cast<int64_t>(static_cast<uint64_t>(S.mul) * static_cast<uint64_t>(x[r]) +
+                                                    static_cast<uint64_t>(S.add));
+                }
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    f[r] = (S.flags & CS_IDENT) ? x[r]
-                                                : static_cast<int64_t>(static_cast<uint64_t>(S.mul) * static_cast<uint64_t>(x[r]) +
-                                                                       static_cast<uint64_t>(S.add));
+                    cur[r] = (fl & CS_CHAIN) ? static_cast<int64_t>(static_cast<uint64_t>(cur[r]) * static_cast<uint64_t>(x[r])) : x[r];
             }
         } else {
 #pragma unroll
-            for (int r = 0; r < R; ++r) f[r] = S.add;
+            for (int r = 0; r < R; ++r)
+                cur[r] = (fl & CS_CHAIN) ? static_cast<int64_t>(static_cast<uint64_t>(cur[r]) * static_cast<uint64_t>(S.add)) : S.add;
         }
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-            cur[r] = (S.flags & CS_CHAIN) ? static_cast<int64_t>(static_cast<uint64_t>(cur[r]) * static_cast<uint64_t>(f[r]))
-                                          : f[r];
-        if (S.acc) {
+        if (!S.acc) continue;
+        // One loop per form of the value's words (uniform across the CTA).
+        const uint32_t off = 4u * P.s32_off[S.acc - 1u];
+        const uint32_t sk = P.s32_kind[S.acc - 1u];
+        if (sk == S32_WIDE) {
             // (Issuing all R low-limb adds before reading any returned value
             // measured slower: more instructions, no latency gained.)
-            const uint32_t w0 = 1u + 2u * (S.acc - 1u);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 if (!((m >> r) & 1u)) continue;
                 const int64_t x = S.kind == VK_COUNT_NZ ? (cur[r] != 0 ? 1 : 0) : cur[r];
-                uint32_t* e = &tab[g[r] * W + w0];
                 const uint32_t xl = static_cast<uint32_t>(x);
-                const uint32_t old = atomicAdd(e, xl);
-                const int32_t add = static_cast<int32_t>(x >> 32) + ((old + xl < old) ? 1 : 0);
-                if (add) atomicAdd(reinterpret_cast<int*>(e + 1), add);
+                const uint32_t old = atom_add_shared(g[r] + off, xl);
+                const uint32_t add = static_cast<uint32_t>(static_cast<int32_t>(x >> 32)) + ((old + xl < old) ? 1u : 0u);
+                if (add) red_add_shared(g[r] + off + 4u, add);
             }
+        } else if (sk == S32_NARROW) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if ((m >> r) & 1u)
+                    red_add_shared(g[r] + off, S.kind == VK_COUNT_NZ ? (cur[r] != 0 ? 1u : 0u) : static_cast<uint32_t>(cur[r]));
+        } else {
+            const uint32_t ref = static_cast<uint32_t>(P.s32_ref[S.acc - 1u]);
+            uint32_t k[R], old[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                k[r] = sk == S32_MIN ? ref - static_cast<uint32_t>(cur[r]) : static_cast<uint32_t>(cur[r]) - ref;
+                if ((m >> r) & 1u) old[r] = lds_u32(g[r] + off);
+                else k[r] = old[r] = 0;
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (k[r] > old[r]) red_max_shared(g[r] + off, k[r]);
         }
     }
 }
