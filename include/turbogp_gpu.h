@@ -345,6 +345,16 @@ TGP_API int tgp_filter(tgp_ctx* ctx, tgp_table_id table, const tgp_pred_node* pr
                uint8_t* bitmap_out, uint32_t* rowids_out, uint64_t rowids_cap,
                uint64_t* count_out);
 
+/* Returns room for `count` u32 words (host or device memory), or NULL. Called
+ * on the calling thread, at most once per call, while the result is still on
+ * the device: it must not call back into this library with the same context. */
+typedef void* (*tgp_alloc_fn)(void* user, uint64_t count);
+
+/* tgp_filter with the row-id buffer allocated once its size is known:
+ * alloc(user, selected rows) is called when at least one row passes. */
+TGP_API int tgp_filter_alloc(tgp_ctx* ctx, tgp_table_id table, const tgp_pred_node* pred, uint32_t npred,
+                     uint8_t* bitmap_out, tgp_alloc_fn alloc, void* user, uint64_t* count_out);
+
 /* ------------------------------------------------------------------------ */
 /* Aggregation queries (scalar, grouped, and join + grouped)                 */
 /* ------------------------------------------------------------------------ */
@@ -514,6 +524,12 @@ TGP_API int tgp_join_probe_pairs(tgp_ctx* ctx, tgp_join_id join, tgp_table_id pr
                          uint32_t probe_key_column, const tgp_pred_node* pred, uint32_t npred,
                          uint32_t* probe_rows, uint32_t* build_rows, uint64_t cap,
                          uint64_t* npairs);
+/* The same pairs into a buffer allocated once their number is known:
+ * alloc(user, 2 x pairs) is called when there is at least one, and receives
+ * every probe row followed by every build row. */
+TGP_API int tgp_join_pairs_alloc(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_table,
+                         uint32_t probe_key_column, const tgp_pred_node* pred, uint32_t npred,
+                         tgp_alloc_fn alloc, void* user, uint64_t* npairs);
 
 /* ------------------------------------------------------------------------ */
 /* Batches: many queries, one persistent launch                              */

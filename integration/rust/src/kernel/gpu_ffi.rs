@@ -268,6 +268,9 @@ pub struct tgp_key_domain {
 // ---------------------------------------------------------------------------
 // Functions
 // ---------------------------------------------------------------------------
+/// Room for `count` u32 words, or null (see `tgp_filter_alloc`).
+pub type tgp_alloc_fn = Option<unsafe extern "C" fn(user: *mut c_void, count: u64) -> *mut c_void>;
+
 extern "C" {
     pub fn tgp_status_string(status: c_int) -> *const c_char;
     pub fn tgp_init(out: *mut *mut tgp_ctx, device: c_int) -> c_int;
@@ -334,6 +337,16 @@ extern "C" {
         rowids_cap: u64,
         count_out: *mut u64,
     ) -> c_int;
+    pub fn tgp_filter_alloc(
+        ctx: *mut tgp_ctx,
+        table: u64,
+        pred: *const tgp_pred_node,
+        npred: u32,
+        bitmap_out: *mut u8,
+        alloc: tgp_alloc_fn,
+        user: *mut c_void,
+        count_out: *mut u64,
+    ) -> c_int;
     pub fn tgp_execute(
         ctx: *mut tgp_ctx,
         q: *const tgp_query,
@@ -398,6 +411,17 @@ extern "C" {
         probe_rows: *mut u32,
         build_rows: *mut u32,
         cap: u64,
+        npairs: *mut u64,
+    ) -> c_int;
+    pub fn tgp_join_pairs_alloc(
+        ctx: *mut tgp_ctx,
+        join: u64,
+        probe_table: u64,
+        probe_key_column: u32,
+        pred: *const tgp_pred_node,
+        npred: u32,
+        alloc: tgp_alloc_fn,
+        user: *mut c_void,
         npairs: *mut u64,
     ) -> c_int;
 

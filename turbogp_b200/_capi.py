@@ -124,6 +124,9 @@ class KernelInfo(C.Structure):
                 ("name", C.c_char_p)]
 
 
+# tgp_alloc_fn: room for `count` u32 words.
+AllocFn = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_uint64)
+
 # (name, restype, argtypes) for every exported symbol of the header.
 PROTOTYPES = [
     ("tgp_status_string", C.c_char_p, [C.c_int]),
@@ -154,6 +157,9 @@ PROTOTYPES = [
      [C.c_void_p, C.c_uint64, C.c_uint32, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     ("tgp_filter", C.c_int,
      [C.c_void_p, C.c_uint64, C.POINTER(PredNode), C.c_uint32, C.c_void_p, C.c_void_p, C.c_uint64,
+      C.POINTER(C.c_uint64)]),
+    ("tgp_filter_alloc", C.c_int,
+     [C.c_void_p, C.c_uint64, C.POINTER(PredNode), C.c_uint32, C.c_void_p, AllocFn, C.c_void_p,
       C.POINTER(C.c_uint64)]),
     ("tgp_execute", C.c_int,
      [C.c_void_p, C.POINTER(Query), C.c_void_p, C.POINTER(AggValue), C.c_uint64, C.POINTER(QueryResult)]),
@@ -192,6 +198,9 @@ PROTOTYPES = [
     ("tgp_join_probe_pairs", C.c_int,
      [C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint32, C.POINTER(PredNode), C.c_uint32, C.c_void_p, C.c_void_p,
       C.c_uint64, C.POINTER(C.c_uint64)]),
+    ("tgp_join_pairs_alloc", C.c_int,
+     [C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint32, C.POINTER(PredNode), C.c_uint32, AllocFn, C.c_void_p,
+      C.POINTER(C.c_uint64)]),
     ("tgp_batch_submit", C.c_int, [C.c_void_p, C.POINTER(BatchItem), C.c_uint32, C.POINTER(C.c_uint64)]),
     ("tgp_batch_poll", C.c_int, [C.c_void_p, C.c_uint64, C.c_int]),
     ("tgp_graph_capture", C.c_int, [C.c_void_p, C.POINTER(Query), C.POINTER(C.c_uint64)]),

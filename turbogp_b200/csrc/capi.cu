@@ -1328,66 +1328,74 @@ int tgp_table_column_stats(tgp_ctx* ctx, tgp_table_id id, uint32_t col, int64_t*
 // --------------------------------------------------------------------------
 static int filter_impl(tgp_ctx* ctx, const Table* T, const tgp_pred_node* pred, uint32_t npred,
                        uint8_t* bitmap_out, uint32_t* rowids_out, uint64_t rowids_cap, uint64_t* count_out,
-                       uint32_t first_words /* >0: only first words into bitmap_out (kernel table) */) {
+                       uint32_t first_words /* >0: only first words into bitmap_out (kernel table) */,
+                       tgp_alloc_fn alloc = nullptr /* row ids go to the buffer it returns */, void* user = nullptr) {
     Builder b(ctx, T);
     TGP_TRY(b.add_pred(pred, npred));
     const uint64_t ntiles = (T->rows + kTileRows - 1) / kTileRows;
     const uint64_t nwords = (T->rows + 31) / 32;
-    const bool need_words = bitmap_out || rowids_out || first_words;
+    const bool rowids = rowids_out || alloc;
+    const bool need_words = bitmap_out || rowids || first_words;
     const uint64_t words = first_words ? std::min<uint64_t>(first_words, nwords) : (need_words ? nwords : 0);
     size_t cub_bytes = 0;
-    if (rowids_out && ntiles) tile_prefix(nullptr, nullptr, ntiles, nullptr, &cub_bytes, ctx->stream);
-    const bool host_rowids = rowids_out && !is_device_ptr(rowids_out);
-    // Host row-id output is compacted into scratch first (worst case: all rows).
-    const uint64_t rowid_scratch = host_rowids ? std::min<uint64_t>(T->rows, rowids_cap) : 0;
+    if (rowids && ntiles) tile_prefix(nullptr, nullptr, ntiles, nullptr, &cub_bytes, ctx->stream);
     Carve cv;
-    TGP_TRY(arena_reserve(ctx, 64 + words * 4 + ntiles * 12 + cub_bytes + rowid_scratch * 4 + 2048, &cv));
-    ScanScratch ss;
-    ss.counters = cv.take<unsigned long long>(4);
-    ss.err = cv.take<uint32_t>(4);
+    TGP_TRY(arena_reserve(ctx, 64 + words * 4 + ntiles * 12 + cub_bytes + 2048, &cv));
+    unsigned long long* block = cv.take<unsigned long long>(6);   // [counters 4][error 2]
     uint32_t* bm = cv.take<uint32_t>(std::max<uint64_t>(words, 1));
     uint32_t* tc = cv.take<uint32_t>(std::max<uint64_t>(ntiles, 1));
     unsigned long long* tb = cv.take<unsigned long long>(std::max<uint64_t>(ntiles, 1));
     void* cub_tmp = cv.take<uint8_t>(cub_bytes + 16);
-    uint32_t* rid_tmp = cv.take<uint32_t>(std::max<uint64_t>(rowid_scratch, 1));
-    TGP_CUDA(cudaMemsetAsync(ss.counters, 0, 32, ctx->stream));
-    TGP_CUDA(cudaMemsetAsync(ss.err, 0, 16, ctx->stream));
+    TGP_CUDA(cudaMemsetAsync(block, 0, 48, ctx->stream));
     if (words) TGP_CUDA(cudaMemsetAsync(bm, 0, words * 4, ctx->stream));
-    if (rowids_out && ntiles) TGP_CUDA(cudaMemsetAsync(tc, 0, ntiles * 4, ctx->stream));
+    if (rowids && ntiles) TGP_CUDA(cudaMemsetAsync(tc, 0, ntiles * 4, ctx->stream));
     Plan& P = b.P;
     P.bitmap = bm;
     P.bitmap_words = static_cast<uint32_t>(std::min<uint64_t>(words, 0xffffffffull));
-    P.tile_counts = rowids_out ? tc : nullptr;
-    P.counters = ss.counters;
-    P.err = ss.err;
+    P.tile_counts = rowids ? tc : nullptr;
+    P.counters = block;
+    P.err = reinterpret_cast<uint32_t*>(block + 4);
     TGP_TRY(size_smem(ctx, P, 0));
     TGP_TRY(launch(ctx, P, MODE_FILTER, false));
-    unsigned long long cnt = 0;
-    uint32_t err = 0;
-    TGP_CUDA(cudaMemcpyAsync(&cnt, ss.counters, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    TGP_CUDA(cudaMemcpyAsync(&err, ss.err, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    // The count comes back first; the prefix of the tiles' counts runs and the
+    // bitmap follows while the host takes it.
+    TGP_TRY(pinned_reserve(ctx, 48));
+    unsigned long long* hb = reinterpret_cast<unsigned long long*>(ctx->hpin);
+    TGP_CUDA(cudaMemcpyAsync(hb, block, 48, cudaMemcpyDeviceToHost, ctx->stream));
     TGP_CUDA(cudaStreamSynchronize(ctx->stream));
-    TGP_TRY(check_kernel_err(ctx, err));
+    const unsigned long long cnt = hb[0];
+    TGP_TRY(check_kernel_err(ctx, static_cast<uint32_t>(hb[4])));
     if (count_out) *count_out = cnt;
     if (first_words) {
         TGP_TRY(copy_out(ctx, bitmap_out, bm, words * 4));
         TGP_CUDA(cudaStreamSynchronize(ctx->stream));
         return TGP_OK;
     }
+    if (rowids && ntiles && cnt) TGP_CUDA(tile_prefix(tc, tb, ntiles, cub_tmp, &cub_bytes, ctx->stream));
     if (bitmap_out) TGP_TRY(copy_out(ctx, bitmap_out, bm, (T->rows + 7) / 8));
-    if (rowids_out) {
-        if (cnt > rowids_cap) {
+    if (rowids) {
+        if (!alloc && cnt > rowids_cap) {
             TGP_CUDA(cudaStreamSynchronize(ctx->stream));
             return fail(ctx, TGP_CAPACITY, "row-id buffer too small");
         }
         if (ntiles && cnt) {
-            TGP_CUDA(tile_prefix(tc, tb, ntiles, cub_tmp, &cub_bytes, ctx->stream));
-            if (!host_rowids) {
-                TGP_CUDA(launch_compact(bm, nwords, ntiles, tb, rowids_out, rowids_cap, ctx->stream));
-            } else {
-                TGP_CUDA(launch_compact(bm, nwords, ntiles, tb, rid_tmp, cnt, ctx->stream));
-                TGP_TRY(copy_out(ctx, rowids_out, rid_tmp, cnt * 4));
+            if (alloc) {
+                rowids_out = static_cast<uint32_t*>(alloc(user, cnt));
+                if (!rowids_out) {
+                    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
+                    return fail(ctx, TGP_OOM, "row-id buffer allocation failed");
+                }
             }
+            uint32_t* dst = rowids_out;
+            uint8_t* tmp = nullptr;
+            if (!is_device_ptr(rowids_out)) {
+                TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&tmp), cnt * 4, "row-id scratch allocation failed"));
+                dst = reinterpret_cast<uint32_t*>(tmp);
+            }
+            cudaError_t e = launch_compact(bm, nwords, ntiles, tb, dst, cnt, ctx->stream);
+            if (e == cudaSuccess && tmp) e = cudaMemcpyAsync(rowids_out, dst, cnt * 4, cudaMemcpyDefault, ctx->stream);
+            dev_free(ctx, tmp);
+            if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("row ids: ") + cudaGetErrorString(e));
         }
     }
     TGP_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1400,6 +1408,15 @@ int tgp_filter(tgp_ctx* ctx, tgp_table_id table, const tgp_pred_node* pred, uint
     const Table* T;
     TGP_TRY(get_table(ctx, table, &T));
     return filter_impl(ctx, T, pred, npred, bitmap_out, rowids_out, rowids_cap, count_out, 0);
+}
+
+int tgp_filter_alloc(tgp_ctx* ctx, tgp_table_id table, const tgp_pred_node* pred, uint32_t npred, uint8_t* bitmap_out,
+                     tgp_alloc_fn alloc, void* user, uint64_t* count_out) {
+    if (!ctx) return TGP_INVALID_ARG;
+    if (!alloc) return fail(ctx, TGP_INVALID_ARG, "null allocation function");
+    const Table* T;
+    TGP_TRY(get_table(ctx, table, &T));
+    return filter_impl(ctx, T, pred, npred, bitmap_out, nullptr, 0, count_out, 0, alloc, user);
 }
 
 // HyperLogLog estimate from 2^14 registers, in the reference's arithmetic
@@ -3885,47 +3902,97 @@ int tgp_join_drop(tgp_ctx* ctx, tgp_join_id id) {
     return TGP_OK;
 }
 
-int tgp_join_probe_pairs(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_table, uint32_t probe_key_column,
-                         const tgp_pred_node* pred, uint32_t npred, uint32_t* probe_rows, uint32_t* build_rows,
-                         uint64_t cap, uint64_t* npairs) {
+static int join_pairs_impl(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_table, uint32_t probe_key_column,
+                           const tgp_pred_node* pred, uint32_t npred, uint32_t* probe_rows, uint32_t* build_rows,
+                           uint64_t cap, tgp_alloc_fn alloc, void* user, uint64_t* npairs) {
     if (!ctx || !npairs) return fail(ctx, TGP_INVALID_ARG, "null argument");
     JoinTable* J;
     TGP_TRY(join_lookup(ctx, join, &J));
     const Table* T;
     TGP_TRY(get_table(ctx, probe_table, &T));
     if (probe_key_column >= T->cols.size()) return fail(ctx, TGP_INVALID_ARG, "probe key column out of range");
+    Plan probe;   // the join table as a probe sees it
+    std::memset(&probe, 0, sizeof(probe));
+    attach_join(probe, *J, 0);
     Builder b(ctx, T);
     TGP_TRY(b.add_pred(pred, npred));
+    Plan& P = b.P;
+    if (b.col2slot[probe_key_column] < 0 && P.nslots >= static_cast<uint32_t>(kMaxSlots))
+        return fail(ctx, TGP_UNSUPPORTED, "query references more than 8 columns");
+    // Selection bitmap (with a WHERE), matches per probe row, then the pairs.
+    const uint64_t words = npred ? (T->rows + 31) / 32 : 0;
+    const size_t ps = pair_scratch(T->rows);
+    Carve cv;
+    TGP_TRY(arena_reserve(ctx, words * 4 + T->rows * 4 + ps + 4096, &cv));
+    unsigned long long* block = cv.take<unsigned long long>(8);   // [counters 4][error][pairs][most]
+    uint32_t* bm = cv.take<uint32_t>(words);
+    PairArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.kept = cv.take<uint32_t>(T->rows);
+    uint8_t* scr = cv.take<uint8_t>(ps);
+    TGP_CUDA(cudaMemsetAsync(block, 0, 64, ctx->stream));
+    P.counters = block;
+    P.err = reinterpret_cast<uint32_t*>(block + 4);
+    if (npred) {
+        P.bitmap = bm;
+        P.bitmap_words = static_cast<uint32_t>(words);
+        TGP_TRY(size_smem(ctx, P, 0));
+        TGP_TRY(launch(ctx, P, MODE_FILTER, false));
+        A.bitmap = bm;
+    }
+    const Column& kc = T->cols[probe_key_column];
+    A.key = kc.dptr;
+    A.dtype = kc.dtype;
+    A.nrows = T->rows;
+    A.tab = probe.jtab;
+    A.mask = probe.jmask;
+    A.log2 = probe.jlog2;
+    A.kmin = probe.jkmin;
+    A.krange = probe.jkrange;
+    A.most = reinterpret_cast<uint32_t*>(block + 6);
+    if (J->empty_range) A.nrows = 0;   // an empty build side matches nothing
+    TGP_CUDA(count_pairs(A, J->wide, J->unique, scr, ps, block + 5, ctx->sms, ctx->stream));
+    unsigned long long hb[8];
+    TGP_CUDA(cudaMemcpyAsync(hb, block, 64, cudaMemcpyDeviceToHost, ctx->stream));
+    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
+    TGP_TRY(check_kernel_err(ctx, static_cast<uint32_t>(hb[4])));
+    const uint64_t n = hb[5];
+    *npairs = n;
+    if (!alloc && n > cap) return fail(ctx, TGP_CAPACITY, "pair buffers too small");
+    if (n == 0) return TGP_OK;
+    if (alloc) {
+        probe_rows = static_cast<uint32_t*>(alloc(user, 2 * n));
+        if (!probe_rows) return fail(ctx, TGP_OOM, "pair buffer allocation failed");
+        build_rows = probe_rows + n;
+    }
+    if (!probe_rows || !build_rows) return fail(ctx, TGP_INVALID_ARG, "null pair buffers");
+    const bool dev_out = is_device_ptr(probe_rows) && is_device_ptr(build_rows);
+    if (static_cast<uint32_t>(hb[6]) <= kPairSortMax) {
+        uint8_t* buf = nullptr;   // the counts stay in the arena while the pairs are written
+        if (!dev_out) TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&buf), n * 8, "join pairs allocation failed"));
+        uint32_t* sp = dev_out ? probe_rows : reinterpret_cast<uint32_t*>(buf);
+        uint32_t* sb = dev_out ? build_rows : sp + n;
+        cudaError_t e = write_pairs(A, J->wide, J->unique, scr, sp, sb, ctx->sms, ctx->stream);
+        if (!dev_out) {
+            const bool one = build_rows == probe_rows + n;
+            if (e == cudaSuccess) e = cudaMemcpyAsync(probe_rows, sp, n * (one ? 8 : 4), cudaMemcpyDefault, ctx->stream);
+            if (e == cudaSuccess && !one) e = cudaMemcpyAsync(build_rows, sb, n * 4, cudaMemcpyDefault, ctx->stream);
+            dev_free(ctx, buf);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("join pairs: ") + cudaGetErrorString(e));
+        return TGP_OK;
+    }
+    // Long runs of one key: the scan engine emits the pairs in any order and
+    // a radix sort orders them.
     int ks;
     TGP_TRY(b.slot_of(probe_key_column, &ks));
-    Plan& P = b.P;
     attach_join(P, *J, ks);
-    // Pass 1 counts pairs (out_cap 0), pass 2 writes them.
-    Carve cv;
-    TGP_TRY(arena_reserve(ctx, 256, &cv));
-    P.counters = cv.take<unsigned long long>(4);
-    P.err = cv.take<uint32_t>(4);
-    P.acc = cv.take<unsigned long long>(2);
-    TGP_CUDA(cudaMemsetAsync(P.counters, 0, 32, ctx->stream));
-    TGP_CUDA(cudaMemsetAsync(P.err, 0, 16, ctx->stream));
-    P.out_pairs = nullptr;
-    P.out_cap = 0;
+    P.bitmap = nullptr;
+    P.bitmap_words = 0;
     TGP_TRY(size_smem(ctx, P, 0));
-    TGP_TRY(launch(ctx, P, MODE_JOIN_PAIRS, false));
-    unsigned long long counters[4];
-    uint32_t err = 0;
-    TGP_CUDA(cudaMemcpyAsync(counters, P.counters, 32, cudaMemcpyDeviceToHost, ctx->stream));
-    TGP_CUDA(cudaMemcpyAsync(&err, P.err, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
-    TGP_TRY(check_kernel_err(ctx, err));
-    const uint64_t n = counters[1];
-    *npairs = n;
-    if (n > cap) return fail(ctx, TGP_CAPACITY, "pair buffers too small");
-    if (n == 0) return TGP_OK;
-    if (!probe_rows || !build_rows) return fail(ctx, TGP_INVALID_ARG, "null pair buffers");
     size_t sort_bytes = 0;
     sort_pairs(nullptr, nullptr, n, nullptr, &sort_bytes, ctx->stream);
-    const bool dev_out = is_device_ptr(probe_rows) && is_device_ptr(build_rows);
     TGP_TRY(arena_reserve(ctx, n * 16 + sort_bytes + (dev_out ? 0 : n * 8) + 1024, &cv));
     unsigned long long* pa = cv.take<unsigned long long>(n);
     unsigned long long* pb = cv.take<unsigned long long>(n);
@@ -3948,11 +4015,24 @@ int tgp_join_probe_pairs(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_tabl
         TGP_TRY(copy_out(ctx, probe_rows, sp, n * 4));
         TGP_TRY(copy_out(ctx, build_rows, sb, n * 4));
     }
+    uint32_t err = 0;
     TGP_CUDA(cudaMemcpyAsync(&err, P.err, 4, cudaMemcpyDeviceToHost, ctx->stream));
     TGP_CUDA(cudaStreamSynchronize(ctx->stream));
     return check_kernel_err(ctx, err);
 }
 
+int tgp_join_probe_pairs(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_table, uint32_t probe_key_column,
+                         const tgp_pred_node* pred, uint32_t npred, uint32_t* probe_rows, uint32_t* build_rows,
+                         uint64_t cap, uint64_t* npairs) {
+    return join_pairs_impl(ctx, join, probe_table, probe_key_column, pred, npred, probe_rows, build_rows, cap, nullptr,
+                           nullptr, npairs);
+}
+
+int tgp_join_pairs_alloc(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_table, uint32_t probe_key_column,
+                         const tgp_pred_node* pred, uint32_t npred, tgp_alloc_fn alloc, void* user, uint64_t* npairs) {
+    if (ctx && !alloc) return fail(ctx, TGP_INVALID_ARG, "null allocation function");
+    return join_pairs_impl(ctx, join, probe_table, probe_key_column, pred, npred, nullptr, nullptr, 0, alloc, user, npairs);
+}
 
 // --------------------------------------------------------------------------
 // Kernel-table boundary (src/kernel/mod.rs)

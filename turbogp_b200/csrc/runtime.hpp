@@ -113,6 +113,32 @@ cudaError_t launch_hll(const uint8_t* col, uint32_t dtype, uint64_t n, const uin
 cudaError_t launch_count_distinct(const unsigned long long* x, uint64_t n, unsigned long long* set,
                                   uint64_t mask, uint32_t log2cap, unsigned long long* counters,
                                   uint32_t* err, int blocks, cudaStream_t st);
+// Join pairs in ascending (probe row, build row) order (join_pairs.cu).
+// count_pairs keeps one word per probe row in `kept`, writes the number of
+// pairs to the device word `total` and raises `most` to the largest number of
+// matches of one row (build sides with repeated keys); write_pairs then
+// writes the pairs (at most kPairSortMax matches per row), with the same
+// scratch of pair_scratch bytes.
+constexpr uint32_t kPairSortMax = 64;
+struct PairArgs {
+    const uint8_t* key;          // probe key column
+    uint32_t dtype;
+    uint32_t log2;               // of the table's slots
+    uint64_t nrows;
+    const uint32_t* bitmap;      // selected probe rows (LSB-first words), null: every row
+    const unsigned long long* tab;
+    uint64_t mask;
+    int64_t kmin;
+    uint64_t krange;             // keys outside [kmin, kmin + krange] match nothing
+    uint32_t* kept;
+    unsigned long long* chunk;   // set by count_pairs
+    uint32_t* most;
+};
+size_t pair_scratch(uint64_t nrows);
+cudaError_t count_pairs(PairArgs A, bool wide, bool unique, void* scratch, size_t scratch_bytes,
+                        unsigned long long* total, int sms, cudaStream_t st);
+cudaError_t write_pairs(const PairArgs& A, bool wide, bool unique, const void* scratch, uint32_t* probe,
+                        uint32_t* build, int sms, cudaStream_t st);
 cudaError_t sort_pairs(const unsigned long long* in, unsigned long long* out, uint64_t n, void* tmp,
                        size_t* tmp_bytes, cudaStream_t st);
 cudaError_t launch_split_pairs(const unsigned long long* pairs, uint64_t n, uint32_t* probe,

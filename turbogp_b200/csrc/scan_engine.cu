@@ -804,10 +804,12 @@ struct Sink {
             for (uint64_t n = 0; n <= P.jmask && !done; ++n) {
                 if (!P.jwide) {
                     // A failed CAS returns the slot's entry: an equal key there
-                    // means the build side has duplicate keys (counter word 3).
+                    // means the build side has duplicate keys (counter word 3,
+                    // a flag: every repeated key adding to it serialised the
+                    // inserts).
                     const unsigned long long old = atomicCAS(P.jtab + h, kEmpty, (rel << 32) | row);
                     done = old == kEmpty;
-                    if (!done && (old >> 32) == rel) atomicAdd(P.counters + 3, 1ull);
+                    if (!done && (old >> 32) == rel) *reinterpret_cast<volatile unsigned long long*>(P.counters + 3) = 1ull;
                 } else if (atomicCAS(P.jtab + 2 * h + 1, 0ull, static_cast<unsigned long long>(row) + 1) == 0ull) {
                     P.jtab[2 * h] = rel;
                     done = true;
