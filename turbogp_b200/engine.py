@@ -11,6 +11,8 @@ back to the CPU.
 from __future__ import annotations
 
 import ctypes as C
+import sys
+import threading
 from dataclasses import dataclass, field
 from typing import Iterable, Sequence
 
@@ -259,6 +261,113 @@ class FilterOutput:
     count: int
     bitmap: np.ndarray | None = None
     rowids: np.ndarray | None = None
+
+
+# ---------------------------------------------------------------------------
+# Result arrays
+# ---------------------------------------------------------------------------
+class _PinnedPool:
+    """Page-locked buffers behind large result arrays. A device-to-host copy
+    into fresh pageable memory runs at the speed at which the host can map and
+    clear pages (a few GB/s on one thread); into a page-locked buffer it runs
+    at link speed. An array holds its buffer until it and every view of it are
+    gone; then the buffer serves the next result. All buffers together stay
+    within LIMIT bytes and the idle ones within KEEP (the rest is unlocked and
+    freed); past LIMIT, or without a device, results are ordinary arrays."""
+
+    MIN = 1 << 20
+    KEEP = 256 << 20
+    LIMIT = 1 << 30
+
+    def __init__(self):
+        self._lock = threading.RLock()   # re-entered when a collection inside a call drops an array
+        self._idle: dict[int, list] = {}
+        self._idle_bytes = self._bytes = 0
+
+    def take(self, nbytes: int) -> np.ndarray | None:
+        """A uint8 array of at least nbytes, or None."""
+        size = 1 << (nbytes - 1).bit_length()
+        with self._lock:
+            free = self._idle.get(size)
+            if free:
+                buf = free.pop()
+                self._idle_bytes -= size
+                return np.asarray(_PinnedLease(self, buf))
+            if self._bytes + size > self.LIMIT:
+                return None
+            self._bytes += size
+        buf = self._register(size)
+        if buf is None:
+            with self._lock:
+                self._bytes -= size
+            return None
+        return np.asarray(_PinnedLease(self, buf))
+
+    @staticmethod
+    def _register(size: int) -> np.ndarray | None:
+        import torch
+        if not torch.cuda.is_available():
+            return None
+        buf = np.empty(size, dtype=np.uint8)
+        if int(torch.cuda.cudart().cudaHostRegister(buf.ctypes.data, size, 1)) != 0:
+            return None
+        return buf
+
+    @staticmethod
+    def _unregister(buf: np.ndarray) -> None:
+        import torch
+        torch.cuda.cudart().cudaHostUnregister(buf.ctypes.data)
+
+    def _give(self, buf: np.ndarray) -> None:
+        with self._lock:
+            if self._idle_bytes + buf.nbytes <= self.KEEP:
+                self._idle.setdefault(buf.nbytes, []).append(buf)
+                self._idle_bytes += buf.nbytes
+                return
+            self._bytes -= buf.nbytes
+        self._unregister(buf)
+
+
+class _PinnedLease:
+    """The owner of one buffer on loan: numpy arrays over it keep it alive."""
+
+    def __init__(self, pool: _PinnedPool, buf: np.ndarray):
+        self._pool, self._buf = pool, buf
+        self.__array_interface__ = {"shape": (buf.nbytes,), "typestr": "|u1", "data": (buf.ctypes.data, False),
+                                    "version": 3}
+
+    def __del__(self):
+        if sys is not None and not sys.is_finalizing():
+            self._pool._give(self._buf)
+
+
+_PINNED = _PinnedPool()
+
+
+def _result_array(n: int, dtype) -> np.ndarray:
+    """An uninitialised array the library writes whole."""
+    nbytes = n * np.dtype(dtype).itemsize
+    if nbytes >= _PinnedPool.MIN:
+        raw = _PINNED.take(nbytes)
+        if raw is not None:
+            return raw[:nbytes].view(dtype)
+    return np.empty(n, dtype=dtype)
+
+
+def _result_words(call) -> np.ndarray:
+    """The u32 result of call(alloc), allocated by the library (tgp_alloc_fn)
+    once its length is known; empty when it allocates nothing."""
+    got = []
+
+    def alloc(_user, count):
+        try:
+            got.append(_result_array(int(count), np.uint32))
+        except Exception:   # the library reports the failed allocation
+            return None
+        return got[-1].ctypes.data
+
+    call(A.AllocFn(alloc))
+    return got[-1] if got else np.empty(0, dtype=np.uint32)
 
 
 # ---------------------------------------------------------------------------
@@ -703,15 +812,15 @@ class Table(Schema):
     def filter(self, where: Pred | None, bitmap: bool = True, rowids: bool = True) -> FilterOutput:
         nodes, n = self.lower_pred(where)
         cnt = C.c_uint64()
-        bm = np.zeros((self.rows + 7) // 8, dtype=np.uint8) if bitmap else None
-        rid = np.zeros(max(1, self.rows), dtype=np.uint32) if rowids else None
-        self.ctx._check(self.ctx.lib.tgp_filter(
-            self.ctx.h, self.id, nodes, n,
-            bm.ctypes.data if bm is not None and bm.size else None,
-            rid.ctypes.data if rid is not None else None,
-            self.rows if rowids else 0, C.byref(cnt)), "tgp_filter")
-        c = int(cnt.value)
-        return FilterOutput(c, bm, rid[:c].copy() if rid is not None else None)
+        bm = _result_array((self.rows + 7) // 8, np.uint8) if bitmap else None
+        bmp = bm.ctypes.data if bm is not None and bm.size else None
+        if not rowids:
+            self.ctx._check(self.ctx.lib.tgp_filter(self.ctx.h, self.id, nodes, n, bmp, None, 0, C.byref(cnt)),
+                            "tgp_filter")
+            return FilterOutput(int(cnt.value), bm, None)
+        ids = _result_words(lambda alloc: self.ctx._check(self.ctx.lib.tgp_filter_alloc(
+            self.ctx.h, self.id, nodes, n, bmp, alloc, None, C.byref(cnt)), "tgp_filter"))
+        return FilterOutput(int(cnt.value), bm, ids)
 
     def prepare(self, aggs: Sequence[Agg], group_by: Sequence[Col | str] = (), where: Pred | None = None,
                 join: "JoinTable | None" = None, probe_key: str | None = None,
@@ -924,18 +1033,11 @@ class JoinTable:
     def probe_pairs(self, probe: Table, probe_key: str, where: Pred | None = None):
         nodes, n = probe.lower_pred(where)
         npairs = C.c_uint64()
-        st = self.ctx.lib.tgp_join_probe_pairs(self.ctx.h, self.id, probe.id, probe.index(probe_key), nodes, n,
-                                               None, None, 0, C.byref(npairs))
-        if st not in (A.OK, A.CAPACITY):
-            self.ctx._check(st, "tgp_join_probe_pairs")
+        rows = _result_words(lambda alloc: self.ctx._check(self.ctx.lib.tgp_join_pairs_alloc(
+            self.ctx.h, self.id, probe.id, probe.index(probe_key), nodes, n, alloc, None, C.byref(npairs)),
+            "tgp_join_probe_pairs"))
         m = int(npairs.value)
-        pr = np.zeros(max(1, m), dtype=np.uint32)
-        br = np.zeros(max(1, m), dtype=np.uint32)
-        if m:
-            self.ctx._check(self.ctx.lib.tgp_join_probe_pairs(
-                self.ctx.h, self.id, probe.id, probe.index(probe_key), nodes, n, pr.ctypes.data, br.ctypes.data, m,
-                C.byref(npairs)), "tgp_join_probe_pairs")
-        return pr[:m], br[:m]
+        return rows[:m], rows[m:]
 
 
 def _flip_side(side: int) -> int:
