@@ -14,6 +14,7 @@
 #include <cub/cub.cuh>
 
 #include "device_common.cuh"
+#include "group_format.cuh"
 #include "plan.hpp"
 #include "turbogp_gpu.h"
 
@@ -567,58 +568,6 @@ __global__ void extract_keys_kernel(const unsigned long long* packed, uint64_t n
     }
 }
 
-// The word of a group's slot that is not zero when the group has rows:
-// [key][count][...] hash slots, one-word slots and direct accumulators.
-__device__ __forceinline__ uint32_t count_word(const HashFormat& F) {
-    return (F.hpack || F.direct_acc) ? 0u : 1u;
-}
-
-// Output group i from its slot s ([key][count][value limbs...], or the direct
-// accumulators' [count lo][count hi][value limbs...]).
-// (key: the slot's packed key word, or its group index.)
-__device__ __forceinline__ void write_group(const unsigned long long* s, unsigned long long key, uint64_t i,
-                                            const HashFormat& F, uint64_t* keys_out, tgp_agg_value* vals_out) {
-    if (keys_out)
-        for (uint32_t k = 0; k < F.nkey; ++k)
-            keys_out[i * F.nkey + k] = static_cast<uint64_t>(F.key_min[k]) +
-                                       (F.direct_acc ? (key / F.key_div[k]) % F.key_mod[k]
-                                                     : (key >> F.key_shift[k]) & F.key_mask[k]);
-    if (!vals_out) return;
-    // One-word slots (F.hpack): the count above `hpack_shift`, below it the
-    // sum of (value - bias) over the slot's rows.
-    const uint64_t cnt = F.hpack ? (F.hpack_shift < 64 ? s[0] >> F.hpack_shift : 0ull) : s[count_word(F)];
-    for (uint32_t a = 0; a < F.nagg; ++a) {
-        tgp_agg_value o;
-        o.count = cnt;
-        if (F.hpack && F.val[a] >= 0) {
-            const uint64_t low = F.hpack_shift ? (s[0] & ((1ull << F.hpack_shift) - 1ull)) : 0ull;
-            const __int128 sum = static_cast<__int128>(low) + static_cast<__int128>(cnt) * F.hpack_bias;
-            o.lo = static_cast<uint64_t>(sum);
-            o.hi = static_cast<int64_t>(sum >> 64);
-            const double f = i128_to_f64_rn(o.lo, o.hi);
-            o.as_f64 = F.func[a] == TGP_AGG_AVG ? (cnt ? f / static_cast<double>(cnt) : 0.0) : f;
-        } else if (F.val[a] < 0) {
-            o.lo = cnt;
-            o.hi = 0;
-            o.as_f64 = static_cast<double>(cnt);
-        } else {
-            const unsigned long long* v = s + 2 + 2 * F.val[a];
-            if (F.kind[a] == VK_MIN || F.kind[a] == VK_MAX) {
-                const int64_t x = static_cast<int64_t>(v[0]);
-                o.lo = static_cast<uint64_t>(x);
-                o.hi = x < 0 ? -1 : 0;
-                o.as_f64 = static_cast<double>(x);
-            } else {
-                o.lo = v[0];
-                o.hi = F.sum64 ? (static_cast<int64_t>(v[0]) >> 63) : static_cast<int64_t>(v[1]);
-                const double f = i128_to_f64_rn(o.lo, o.hi);
-                o.as_f64 = F.func[a] == TGP_AGG_AVG ? (cnt ? f / static_cast<double>(cnt) : 0.0) : f;
-            }
-        }
-        vals_out[i * F.nagg + a] = o;
-    }
-}
-
 __global__ void format_hash_groups_kernel(const unsigned long long* packed, const uint32_t* order, uint64_t n,
                                           const HashFormat F, uint64_t* keys_out, tgp_agg_value* vals_out) {
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
@@ -734,7 +683,7 @@ cudaError_t count_direct_groups(const unsigned long long* htab, uint64_t nslots,
     cudaError_t e = cudaMemsetAsync(counts + nb, 0, 8, st);
     if (e != cudaSuccess) return e;
     if (nb) count_direct_kernel<<<static_cast<unsigned>(nb), kAuxThreads, 0, st>>>(
-            htab, nslots, F.hstride, (F.hpack || F.direct_acc) ? 0u : 1u, counts);
+            htab, nslots, F.hstride, count_word(F), counts);
     e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, offsets, static_cast<int>(nb + 1), st);
     if (e != cudaSuccess) return e;
     return cudaMemcpyAsync(total, offsets + nb, 8, cudaMemcpyDeviceToDevice, st);

@@ -818,6 +818,48 @@ int launch_direct_groups(tgp_ctx* ctx, const Plan& P, uint64_t max_abs_val) {
     return TGP_OK;
 }
 
+// GROUP BY of one sparse key into 16-byte hash slots: the streaming kernel of
+// groupby_direct.cu in place of the scan pipeline (one CTA of 17 warps per SM,
+// a row's dependent table accesses one after another).
+int launch_hash_groups(tgp_ctx* ctx, const Plan& P, uint64_t max_abs_val) {
+    const bool hasv = P.nval != 0;
+    HashGroupArgs A;
+    std::memset(&A, 0, sizeof(A));
+    for (uint32_t i = 0; i < P.nleaf; ++i) {
+        A.leaf_col[i] = P.slot[P.leaf[i].slot].ptr;
+        A.leaf_lo[i] = P.leaf[i].lo32;
+        A.leaf_sp[i] = P.leaf[i].span32;
+        if (P.leaf[i].negate) A.leaf_neg |= 1u << i;
+    }
+    A.nleaf = P.nleaf;
+    A.key = P.slot[P.gkey[0].slot].ptr;
+    A.val = hasv ? P.slot[P.val[0].f[0].slot].ptr : nullptr;
+    A.nrows = P.nrows;
+    A.kmin = P.gkey[0].min;
+    A.mul = hasv ? P.val[0].f[0].mul : 1;
+    A.add = hasv ? P.val[0].f[0].add : 0;
+    A.ident = A.mul == 1 && A.add == 0;
+    A.nz = hasv && P.val[0].kind == VK_COUNT_NZ;
+    const unsigned __int128 rows_cta = hash_group_rows_per_cta(P.nrows, ctx->sms);
+    A.hs = P.hsm_slots && rows_cta * std::max<uint64_t>(max_abs_val, 1) < (static_cast<unsigned __int128>(1) << 31);
+    A.log2 = P.hlog2;
+    A.shift = P.hpack_shift;
+    A.mask = static_cast<uint32_t>(P.hmask);
+    A.probes = static_cast<uint32_t>(std::min<uint64_t>(P.hprobes, 0xffffffffull));
+    A.bias = P.hpack_bias;
+    A.one = (1ull << P.hpack_shift) - static_cast<uint64_t>(P.hpack_bias);
+    A.slots = P.htab;
+    A.err = P.err;
+    A.counters = P.counters;
+    const uint32_t kdt = P.slot[P.gkey[0].slot].dtype, vdt = hasv ? P.slot[P.val[0].f[0].slot].dtype : 0u;
+    std::pair<cudaEvent_t, cudaEvent_t>* ev = nullptr;
+    TGP_TRY(profile_begin(ctx, &ev));
+    const cudaError_t e = launch_hash_group(A, kdt, vdt, ctx->sms, ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("group launch: ") + cudaGetErrorString(e));
+    if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
+    return TGP_OK;
+}
+
 // The TPC-H Q1 shape (two u8 keys, the fixed value program ShapeQ1) under at
 // most four int32 predicate leaves and no join: the streaming kernel of
 // groupby_direct.cu in place of the scan pipeline when every global sum and
@@ -1957,6 +1999,7 @@ static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t s
             P.hlog2 = log2u(hcap);
             P.hmask = hcap - 1;
         }
+        P.hprobes = hcap;
     }
     // One staged key and at most two SUM / COUNT(col) values of one staged
     // factor each: the column path of global / hash grouping.
@@ -2013,24 +2056,33 @@ static void bound_presum(tgp_ctx* ctx, QueryState& qs) {
     if (bound >= (static_cast<unsigned __int128>(1) << 31)) P.hsm_slots = 0;
 }
 
-// A directly indexed table of COUNT(*) and at most one SUM / COUNT(col)
-// whose fields provably never meet takes one-word slots (Plan::hpack): the
-// count in the top bits (enough for every row), the sum of (value - its
-// minimum) below. Groups formatted straight from the table only (no top-N,
-// at most kMaxFormatAggs aggregates).
+// ORDER BY one aggregate, LIMIT n (tgp_execute_topn).
+struct TopNReq {
+    uint32_t agg;
+    bool desc;
+    uint64_t limit;
+};
+
+// A group table of one key with COUNT(*) and at most one SUM / COUNT(col) whose
+// fields provably never meet holds them in one word (Plan::hpack): the count
+// in the top bits (enough for every row), the sum of (value - its minimum)
+// below. Groups formatted on the device only (top-N: through the selection,
+// whose ordering values are int64).
 //
 // Direct accumulators in global memory (MODE_GROUP_GLOBAL, placed there by
 // the planner's rule) move to one-word slots on the same conditions: a slot
 // is 8 bytes instead of 32 or 48 and a row's global update one add instead
-// of two (40M rows, 500K Zipf(1.1) keys: accumulate, clear and read the
-// table 316 us -> see the streaming kernel's figures).
-static void plan_one_word_slots(QueryState& qs, const tgp_query* q, bool topn) {
+// of two (40M rows over 500K Zipf(1.1) keys: scan kernel 316 us, streaming
+// kernel on one-word slots 154 us). Hash slots shrink from 48 to 16 bytes.
+static void plan_one_word_slots(QueryState& qs, const tgp_query* q, const TopNReq* tn) {
     Plan& P = qs.b->P;
     const Builder& b = *qs.b;
     const bool global = qs.mode == MODE_GROUP_GLOBAL && qs.kn.placement == 0;
-    if (!(((qs.mode == MODE_GROUP_HASH && P.hdirect) || global) && P.hash_fast && P.nval <= 1 && !topn &&
+    const bool hashed = qs.mode == MODE_GROUP_HASH && !P.hdirect;
+    if (!((qs.mode == MODE_GROUP_HASH || global) && P.hash_fast && P.nval <= 1 &&
+          (!tn || (P.sum64 && tn->limit >= 1 && tn->limit <= kTopSelectMax)) &&
           q->nagg <= static_cast<uint32_t>(kMaxFormatAggs) && P.ngkey == 1 && P.gkey[0].shift == 0 &&
-          (!P.hsm_slots || P.hsm_key32) && (P.nval == 0 || !b.val_big[0])))
+          (hashed || !P.hsm_slots || P.hsm_key32) && (P.nval == 0 || !b.val_big[0])))
         return;
     const uint64_t rows = std::max<uint64_t>(qs.T->rows, 1);
     const uint32_t cbits = 64u - static_cast<uint32_t>(__builtin_clzll(rows));  // count <= rows < 2^cbits
@@ -2042,7 +2094,7 @@ static void plan_one_word_slots(QueryState& qs, const tgp_query* q, bool topn) {
         P.hpack = 1;
         P.hpack_shift = shift;
         P.hpack_bias = P.nval ? static_cast<int64_t>(b.val_lo[0]) : 0;
-        P.hstride = 1;
+        P.hstride = hashed ? 2 : 1;
         if (global) {
             qs.mode = MODE_GROUP_HASH;
             qs.hcap = std::max<uint64_t>(16, qs.ngroups_direct);
@@ -2096,13 +2148,6 @@ static int decode_direct(tgp_ctx* ctx, const QueryState& qs, const unsigned long
         return TGP_OK;
     }
 
-// ORDER BY one aggregate, LIMIT n (tgp_execute_topn).
-struct TopNReq {
-    uint32_t agg;
-    bool desc;
-    uint64_t limit;
-};
-
 // Keeps the first min(limit, n) of n decoded groups in the order of one
 // aggregate's exact value (AVG: its f64), ties in the given (key) order.
 static void host_topn(const TopNReq& tn, uint32_t nkey, uint32_t nagg, const std::vector<uint64_t>& keys,
@@ -2129,6 +2174,51 @@ static void host_topn(const TopNReq& tn, uint32_t nkey, uint32_t nagg, const std
     result->ngroups = m;
 }
 
+// A group hash table is sized by a bound on the distinct keys, the rows when
+// nothing better is known: 20M rows over 1M ids took a table of 32M 48-byte
+// slots (1.6 GB), filled in 0.27 ms, probed out of L2 and searched for its
+// 480K groups in 0.63 ms. Large tables are sized instead from a sketch of the
+// keys (one pass over the key columns; the WHERE only lowers the number):
+// half again the estimate, to a power of two. A row that finds no slot within
+// kSketchProbes raises kErrHashFull and the query runs again on the full
+// table, so the estimate decides speed only. Below kSketchMinTable the pass and
+// its wait cost what the smaller table saves.
+constexpr size_t kSketchMinTable = 64u << 20;
+constexpr uint64_t kSketchProbes = 1024;
+
+static int shrink_group_table(tgp_ctx* ctx, QueryState& qs, bool* shrunk) {
+    Plan& P = qs.b->P;
+    *shrunk = false;
+    if (qs.mode != MODE_GROUP_HASH || P.hdirect || qs.hcap * P.hstride * 8 < kSketchMinTable) return TGP_OK;
+    SketchArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.nkey = P.ngkey;
+    for (uint32_t k = 0; k < P.ngkey; ++k) {
+        if (P.gkey[k].build_side) return TGP_OK;
+        A.col[k] = P.slot[P.gkey[k].slot].ptr;
+        A.dtype[k] = P.gkey[k].dtype;
+        A.min[k] = P.gkey[k].min;
+        A.shift[k] = P.gkey[k].shift;
+    }
+    A.nrows = P.nrows;
+    Carve cv;
+    TGP_TRY(arena_reserve(ctx, key_sketch_bytes(), &cv));
+    A.regs = cv.take<uint32_t>(key_sketch_bytes() / 4);
+    TGP_TRY(pinned_reserve(ctx, key_sketch_bytes()));
+    TGP_CUDA(launch_key_sketch(A, ctx->sms, ctx->stream));
+    TGP_CUDA(cudaMemcpyAsync(ctx->hpin, A.regs, key_sketch_bytes(), cudaMemcpyDeviceToHost, ctx->stream));
+    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
+    const double est = key_sketch_estimate(reinterpret_cast<const uint32_t*>(ctx->hpin));
+    const uint64_t want = next_pow2(1024 + static_cast<uint64_t>(est * 1.5));
+    if (want >= qs.hcap) return TGP_OK;
+    qs.hcap = want;
+    P.hlog2 = log2u(want);
+    P.hmask = want - 1;
+    P.hprobes = std::min<uint64_t>(want, kSketchProbes);
+    *shrunk = true;
+    return TGP_OK;
+}
+
 // Whether a run of the query formats its groups on the device straight from
 // their table: directly indexed slots, and direct accumulators of many groups
 // (few are decoded on the host from the one readback that carries the
@@ -2140,13 +2230,15 @@ static bool formats_direct(const QueryState& qs, const tgp_query* q) {
 }
 
 static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tgp_agg_value* vals_out,
-                        uint64_t group_cap, tgp_query_result* result, const TopNReq* tn) {
+                        uint64_t group_cap, tgp_query_result* result, const TopNReq* tn, bool full_table = false) {
     if (!ctx || !q || !result) return fail(ctx, TGP_INVALID_ARG, "null argument");
     std::memset(result, 0, sizeof(*result));
     if (tn && tn->agg >= q->nagg) return fail(ctx, TGP_INVALID_ARG, "ORDER BY aggregate index out of range");
     QueryState qs;
     TGP_TRY(plan_query(ctx, q, qs, scan_kernel_static_smem()));
-    plan_one_word_slots(qs, q, tn != nullptr);
+    plan_one_word_slots(qs, q, tn);
+    bool shrunk = false;
+    if (!full_table) TGP_TRY(shrink_group_table(ctx, qs, &shrunk));
     Builder& b = *qs.b;
     Plan& P = b.P;
     const Table* T = qs.T;
@@ -2193,7 +2285,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     } else {
         TGP_CUDA(cudaMemsetAsync(block, 0, block_words * 8, ctx->stream));
     }
-    if (mode == MODE_GROUP_HASH && P.hpack) {
+    if (mode == MODE_GROUP_HASH && P.hpack && P.hdirect) {
         TGP_CUDA(cudaMemsetAsync(P.htab, 0, hcap * 8, ctx->stream));
     } else if (mode == MODE_GROUP_HASH) {
         // Keys EMPTY, counters 0, value limbs: MIN/MAX identity or 0 (one pass).
@@ -2209,7 +2301,11 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     }
     TGP_TRY(size_smem(ctx, P, extra, scan_kernel_static_smem(), &qs.kn));
     bound_presum(ctx, qs);
-    if (P.hpack && P.nleaf == 0 && P.hash_fast && !ctx->dbg_skip_tile1 &&
+    const bool streams = P.hpack && P.hash_fast && !ctx->dbg_skip_tile1;
+    if (streams && !P.hdirect && hcap <= (1ull << 32) && P.nleaf <= 4 && (P.nleaf == 0 || (P.all_and && P.kend[0] == P.nleaf)) &&
+        hash_group_supported(P.slot[P.gkey[0].slot].dtype, P.nval ? P.slot[P.val[0].f[0].slot].dtype : 0u)) {
+        TGP_TRY(launch_hash_groups(ctx, P, b.max_abs_val));
+    } else if (streams && P.hdirect && P.nleaf == 0 &&
         direct_group_supported(P.slot[P.gkey[0].slot].dtype, P.nval ? P.slot[P.val[0].f[0].slot].dtype : 0u)) {
         TGP_TRY(launch_direct_groups(ctx, P, b.max_abs_val));
     } else {
@@ -2257,12 +2353,81 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         TGP_CUDA(count_direct_groups(table, fmt_slots, group_format(), fmt, fmt_scratch, P.counters + 2, ctx->stream));
     }
 
+    // Top-N of many groups by selection: the groups are listed and narrowed
+    // behind the scan, and one wait brings the counters and the result.
+    TopNSpec S;
+    std::memset(&S, 0, sizeof(S));
+    if (tn) {
+        S.val = amap[tn->agg].val;
+        S.kind = static_cast<uint8_t>(S.val >= 0 ? P.val[S.val].kind : VK_SUM);
+        S.func = static_cast<uint8_t>(amap[tn->agg].func);
+        S.desc = tn->desc ? 1 : 0;
+        S.sum64 = P.sum64 ? 1 : 0;
+    }
+    const bool one_word = S.val < 0 || S.kind == VK_MIN || S.kind == VK_MAX || S.func == TGP_AGG_AVG || S.sum64;
+    if (tn && one_word && tn->limit >= 1 && tn->limit <= kTopSelectMax && nagg <= static_cast<uint32_t>(kMaxFormatAggs) &&
+        q->ngroup && (mode == MODE_GROUP_HASH || ngroups_direct >= kDeviceFormatGroups)) {
+        const bool indexed = mode != MODE_GROUP_HASH || P.hdirect;
+        const uint64_t nslots = mode == MODE_GROUP_HASH ? hcap : ngroups_direct;
+        uint64_t max_groups = static_cast<uint64_t>(std::min<unsigned __int128>(D, nslots));
+        if (!q->join) max_groups = std::min<uint64_t>(max_groups, std::max<uint64_t>(T->rows, 1));
+        const HashFormat F = group_format();
+        const size_t kb = (static_cast<size_t>(tn->limit) * q->ngroup * 8 + 255) & ~size_t{255};
+        const size_t vb = static_cast<size_t>(tn->limit) * nagg * sizeof(tgp_agg_value);
+        const size_t out = 256 + kb + vb, sb = top_select_scratch(max_groups);
+        uint8_t* buf = nullptr;
+        TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&buf), ((out + 255) & ~size_t{255}) + sb, "top-N allocation failed"));
+        uint8_t* scr = buf + ((out + 255) & ~size_t{255});
+        int st = pinned_reserve(ctx, 64 + out);
+        cudaError_t e = st == TGP_OK ? top_select_begin(table, nslots, F, indexed, S, tn->limit,
+                                                        indexed ? log2u(next_pow2(nslots)) : total_bits, scr, ctx->sms,
+                                                        ctx->stream)
+                                     : cudaSuccess;
+        TopState state;
+        std::memset(&state, 0, sizeof(state));
+        uint32_t err = 0;
+        unsigned long long selected = 0;
+        for (uint32_t round = 0; st == TGP_OK && e == cudaSuccess && !state.done; ++round) {
+            if (round == 32) {
+                st = fail(ctx, TGP_DEVICE_ERROR, "top-N selection did not finish");
+                break;
+            }
+            e = top_select_narrow(table, max_groups, round, F, tn->limit, scr, reinterpret_cast<uint64_t*>(buf + 256),
+                                  reinterpret_cast<tgp_agg_value*>(buf + 256 + kb), ctx->sms, ctx->stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(buf, scr, sizeof(TopState), cudaMemcpyDeviceToDevice, ctx->stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->hpin, block, 48, cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->hpin + 64, buf, out, cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+            if (e != cudaSuccess) break;
+            const unsigned long long* hw = reinterpret_cast<const unsigned long long*>(ctx->hpin);
+            selected = hw[0];
+            err = static_cast<uint32_t>(hw[4]);
+            if (err & (kErrWaitTimeout | kErrHashFull)) break;
+            std::memcpy(&state, ctx->hpin + 64, sizeof(state));
+        }
+        dev_free(ctx, buf);
+        if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("top-N: ") + cudaGetErrorString(e));
+        if (st != TGP_OK) return st;
+        if (shrunk && (err & kErrHashFull) && !(err & kErrWaitTimeout))
+            return execute_impl(ctx, q, keys_out, vals_out, group_cap, result, tn, true);
+        TGP_TRY(check_kernel_err(ctx, err));
+        result->rows_scanned = T->rows;
+        result->rows_selected = selected;
+        result->flags = (err & kErrRowOverflow) ? TGP_RESULT_ROW_OVERFLOW : 0u;
+        result->ngroups = std::min<uint64_t>(tn->limit, state.total);
+        if (keys_out) std::memcpy(keys_out, ctx->hpin + 64 + 256, result->ngroups * q->ngroup * 8);
+        if (vals_out) std::memcpy(vals_out, ctx->hpin + 64 + 256 + kb, result->ngroups * nagg * sizeof(tgp_agg_value));
+        return TGP_OK;
+    }
+
     TGP_TRY(pinned_reserve(ctx, back_words * 8));
     TGP_CUDA(cudaMemcpyAsync(ctx->hpin, block, back_words * 8, cudaMemcpyDeviceToHost, ctx->stream));
     TGP_CUDA(cudaStreamSynchronize(ctx->stream));
     const unsigned long long* hb = reinterpret_cast<const unsigned long long*>(ctx->hpin);
     unsigned long long counters[4] = {hb[0], hb[1], hb[2], hb[3]};
     const uint32_t err = static_cast<uint32_t>(hb[4] & 0xffffffffull);
+    if (shrunk && (err & kErrHashFull) && !(err & kErrWaitTimeout))
+        return execute_impl(ctx, q, keys_out, vals_out, group_cap, result, tn, true);
     TGP_TRY(check_kernel_err(ctx, err));
 
     result->rows_scanned = T->rows;
@@ -2348,13 +2513,6 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         tgp_agg_value* dvals = vbytes ? reinterpret_cast<tgp_agg_value*>(buf + vofs) : nullptr;
         cudaError_t e;
         if (tn) {
-            TopNSpec S;
-            std::memset(&S, 0, sizeof(S));
-            S.val = amap[tn->agg].val;
-            S.kind = static_cast<uint8_t>(S.val >= 0 ? P.val[S.val].kind : VK_SUM);
-            S.func = static_cast<uint8_t>(amap[tn->agg].func);
-            S.desc = tn->desc ? 1 : 0;
-            S.sum64 = P.sum64 ? 1 : 0;
             e = topn_hash_groups(packed, ng, F, total_bits, S, nout, buf, sbytes, dkeys, dvals, ctx->sms, ctx->stream);
             result->ngroups = nout;
         } else {
@@ -2419,7 +2577,7 @@ int tgp_query_footprint(tgp_ctx* ctx, const tgp_query* q, uint64_t* device_bytes
     if (!ctx || !q || !device_bytes) return fail(ctx, TGP_INVALID_ARG, "null argument");
     QueryState qs;
     TGP_TRY(plan_query(ctx, q, qs, scan_kernel_static_smem(), nullptr, /*dry=*/true));
-    plan_one_word_slots(qs, q, false);
+    plan_one_word_slots(qs, q, nullptr);
     const Plan& P = qs.b->P;
     // What execute_impl carves or allocates for one run of the query.
     uint64_t bytes = qs.block_words() * 8 + 1024 + qs.pending_dev_bytes;

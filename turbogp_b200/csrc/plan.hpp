@@ -223,6 +223,8 @@ struct alignas(16) Plan {
     // Group hash table (MODE_GROUP_HASH): slot = [key][count][v0 lo][v0 hi]...
     unsigned long long* htab;
     uint64_t hmask;
+    uint64_t hprobes;       // probes before a row gives up with kErrHashFull (the slots, or a short bound on a
+                            // table sized from a sketch of the keys)
     uint32_t hlog2;
     uint32_t hstride;       // u64 words per slot
     uint32_t hsm_slots;     // per-CTA shared pre-aggregation slots (power of two; 0 = none):
@@ -274,12 +276,12 @@ struct alignas(16) Plan {
     // row's update needs no probe, no compare and no claim; a slot whose
     // count is not zero is occupied (its key word stays empty).
     uint32_t hdirect;
-    // One-word direct slots (MODE_GROUP_HASH, hdirect, hstride = 1): a slot
-    // holds (row count << hpack_shift) + the sum of (value - hpack_bias) over
-    // its rows, both fields proven by the host never to carry into the other
-    // (rows < 2^(64 - hpack_shift), rows x value range < 2^hpack_shift), so a
-    // row is one non-returning 64-bit add and the table is a quarter of the
-    // [key][count][lo][hi] layout's size. 0 = that layout.
+    // One-word groups (MODE_GROUP_HASH): a word holds (row count <<
+    // hpack_shift) + the sum of (value - hpack_bias) over its rows, both
+    // fields proven by the host never to carry into the other (rows <
+    // 2^(64 - hpack_shift), rows x value range < 2^hpack_shift), so a row is
+    // one non-returning 64-bit add. A direct slot is that word (hstride 1), a
+    // hash slot [key][word] (hstride 2). 0 = the [key][count][lo][hi] layout.
     uint32_t hpack;
     uint32_t hpack_shift;
     int64_t hpack_bias;
@@ -359,7 +361,7 @@ struct SlotImage {
 constexpr int kMaxFormatAggs = 32;
 struct HashFormat {
     uint32_t nkey, nagg, hstride, sum64;  // sum64: value limbs hold int64 sums (hi = sign of lo)
-    uint32_t hpack, hpack_shift;          // one-word direct slots (Plan::hpack)
+    uint32_t hpack, hpack_shift;          // one-word groups (Plan::hpack)
     int64_t hpack_bias;
     // Direct-indexed accumulators ([count lo][count hi][v0 lo][v0 hi]...,
     // hstride words per group): key k of group index g is

@@ -64,6 +64,33 @@ struct Q1Args {
     unsigned long long* acc;
     unsigned long long* counters;
 };
+// GROUP BY one sparse key into 16-byte hash slots [key][count << shift + sum]
+// under at most four int32 leaves (groupby_direct.cu). hs: keep the per-CTA
+// shared table (no CTA's i32 partial can reach 2^31 over
+// hash_group_rows_per_cta rows).
+struct HashGroupArgs {
+    const uint8_t* leaf_col[4];
+    uint32_t leaf_lo[4], leaf_sp[4];
+    uint32_t leaf_neg, nleaf;
+    const uint8_t* key;
+    const uint8_t* val;            // null: COUNT(*) only
+    uint64_t nrows;
+    int64_t kmin;
+    int64_t mul, add;
+    uint32_t ident, nz;
+    uint32_t hs, hs_log2;
+    uint32_t log2, shift;          // of the slots (at most 2^32), of the word's count
+    uint32_t mask, probes;
+    unsigned long long one;
+    int64_t bias;
+    unsigned long long* slots;
+    uint32_t* err;
+    unsigned long long* counters;  // [0] += selected rows
+};
+bool hash_group_supported(uint32_t kdt, uint32_t vdt);
+uint64_t hash_group_grid(uint64_t nrows, int sms);
+uint64_t hash_group_rows_per_cta(uint64_t nrows, int sms);
+cudaError_t launch_hash_group(const HashGroupArgs& A, uint32_t kdt, uint32_t vdt, int sms, cudaStream_t st);
 size_t q1_group_smem(uint32_t ngroups);
 int q1_group_ctas_per_sm(uint32_t ngroups);
 cudaError_t launch_q1_group(const Q1Args& A, int grid, cudaStream_t st);
@@ -166,6 +193,39 @@ cudaError_t format_direct_groups(const unsigned long long* htab, uint64_t nslots
 cudaError_t topn_hash_groups(const unsigned long long* packed, uint64_t n, const HashFormat& F, uint32_t key_bits,
                              const TopNSpec& S, uint64_t limit, void* scratch, size_t scratch_bytes,
                              uint64_t* keys_out, tgp_agg_value* vals_out, int sms, cudaStream_t st);
+// Distinct-count sketch of packed probe-side group keys (group_select.cu):
+// the registers (key_sketch_bytes) are read back and estimated on the host.
+struct SketchArgs {
+    uint32_t nkey;
+    uint32_t dtype[kMaxGroupKeys];
+    const uint8_t* col[kMaxGroupKeys];
+    int64_t min[kMaxGroupKeys];
+    uint8_t shift[kMaxGroupKeys];
+    uint64_t nrows;
+    uint32_t* regs;
+};
+size_t key_sketch_bytes();
+cudaError_t launch_key_sketch(const SketchArgs& A, int sms, cudaStream_t st);
+double key_sketch_estimate(const uint32_t* regs);
+// The first `limit` (at most kTopSelectMax) groups of a hash table, a directly
+// indexed table or direct accumulators in the order of one aggregate (ties in
+// ascending key order), formatted like format_hash_groups. Ordering values of
+// one word only (no int128 sums). begin lists the groups, each narrow (round
+// 0, 1, ...) launches one selection step; TopState::done says that the groups
+// are written and TopState::total how many there are. The state is the first
+// bytes of the scratch.
+constexpr uint64_t kTopSelectMax = 1024;
+struct TopState {
+    unsigned long long n, lo, hi, want, key_hi, nnext, total;
+    uint32_t bucket, nsure, by_key, done;
+};
+size_t top_select_scratch(uint64_t max_groups);
+cudaError_t top_select_begin(const unsigned long long* htab, uint64_t nslots, const HashFormat& F, bool direct,
+                             const TopNSpec& S, uint64_t limit, uint32_t key_bits, void* scratch, int sms,
+                             cudaStream_t st);
+cudaError_t top_select_narrow(const unsigned long long* htab, uint64_t max_groups, uint32_t round, const HashFormat& F,
+                              uint64_t limit, void* scratch, uint64_t* keys_out, tgp_agg_value* vals_out, int sms,
+                              cudaStream_t st);
 // One thread that spins on %globaltimer for `ns` nanoseconds (at most 1 ms).
 cudaError_t launch_delay(uint64_t ns, cudaStream_t st);
 // Device-to-host copy by a kernel into page-locked (mapped) host memory; both

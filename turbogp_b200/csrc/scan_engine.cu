@@ -509,8 +509,10 @@ __device__ __forceinline__ unsigned long long* hash_group_slot(const Plan& P, ui
         return P.htab + key * P.hstride;
     }
     uint64_t h = hash_slot(key, P.hlog2);
-    for (uint64_t n = 0; n <= P.hmask; ++n) {
+    for (uint64_t n = 0; n < P.hprobes; ++n) {
         unsigned long long* s = P.htab + h * P.hstride;
+        // A table that overflowed is given up: no row probes it to the end.
+        if ((n & 31u) == 31u && (*reinterpret_cast<volatile uint32_t*>(P.err) & kErrHashFull)) return nullptr;
         unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(s);
         if (k == kEmpty) k = atomicCAS(s, kEmpty, key);
         if (k == kEmpty || k == key) return s;
@@ -520,16 +522,14 @@ __device__ __forceinline__ unsigned long long* hash_group_slot(const Plan& P, ui
     return nullptr;
 }
 
-// Adds `cnt` rows whose value arguments sum to `xsum` to the one-word direct
-// slot of `key` (P.hpack): one non-returning 64-bit add of
+// Adds `cnt` rows whose value arguments sum to `xsum` to the one-word group of
+// `key` (P.hpack): one non-returning 64-bit add of
 // (cnt << shift) + (xsum - cnt * bias).
 __device__ __forceinline__ void hpack_add(const Plan& P, uint64_t key, uint64_t cnt, int64_t xsum) {
-    if (key > P.hmask) {
-        atomicOr(P.err, kErrHashFull);
-        return;
-    }
-    atomicAdd(P.htab + key, (cnt << P.hpack_shift) +
-                                (static_cast<unsigned long long>(xsum) - cnt * static_cast<uint64_t>(P.hpack_bias)));
+    unsigned long long* slot = hash_group_slot(P, key);
+    if (slot == nullptr) return;
+    atomicAdd(slot + (P.hdirect ? 0 : 1),
+              (cnt << P.hpack_shift) + (static_cast<unsigned long long>(xsum) - cnt * static_cast<uint64_t>(P.hpack_bias)));
 }
 
 // This CTA's shared pre-aggregation table (P.hsm_slots slots: keys, u32
@@ -1762,6 +1762,10 @@ __device__ __forceinline__ void hash_fast_tile(const Plan& P, uint8_t* extra, co
     for (int r = 0; r < R; ++r) {
         if (!((pend >> r) & 1u)) continue;
         unsigned long long* base;
+        if (MODE == MODE_GROUP_HASH && P.hpack) {
+            hpack_add(P, key[r], 1, P.nval ? x[r][0] : 0);
+            continue;
+        }
         if (MODE == MODE_GROUP_HASH) {
             unsigned long long* slot = hash_group_slot(P, key[r]);
             if (slot == nullptr) continue;
@@ -2006,7 +2010,7 @@ __device__ __forceinline__ void process_tile(const Plan& P, Sink<MODE, ACC128, N
     if constexpr (MODE == MODE_GROUP_HASH || MODE == MODE_GROUP_GLOBAL) {
         if (!TAIL && P.hash_fast) {
             if constexpr (MODE == MODE_GROUP_HASH) {
-                if (P.hpack) {
+                if (P.hpack && P.hdirect) {
                     hpack_tile<R>(P, extra, stage, t, m);
                     return;
                 }
