@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -144,6 +146,62 @@ int pinned_reserve(tgp_ctx* ctx, size_t bytes) {
         return fail(ctx, TGP_OOM, "pinned host allocation failed");
     }
     ctx->hpin_cap = want;
+    return TGP_OK;
+}
+
+// Result blocks up to this size are handed over by the kernel itself.
+constexpr size_t kHandoverBytes = 256u << 10;
+
+// Prepares the handover of a result block of `words` words: its device block
+// (zero, 16-byte aligned) and the ResultOut of the launch. Allocates once per
+// context; without the memory the caller clears and copies as for larger
+// blocks (out->host stays null).
+int handover_begin(tgp_ctx* ctx, uint64_t words, ResultOut* out) {
+    std::memset(out, 0, sizeof(*out));
+    if (words * 8 > kHandoverBytes) return TGP_OK;
+    if (!ctx->rblock) {
+        void *d = nullptr, *h = nullptr;
+        if (cudaMalloc(&d, kHandoverBytes + 256) != cudaSuccess ||
+            cudaHostAlloc(&h, kHandoverBytes + 256, cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            if (d) cudaFree(d);
+            return TGP_OK;
+        }
+        std::memset(h, 0, kHandoverBytes + 256);
+        ctx->rblock = static_cast<unsigned long long*>(d);
+        ctx->rhost = static_cast<unsigned long long*>(h);
+        ctx->rdirty = true;
+    }
+    if (ctx->rdirty) TGP_CUDA(cudaMemsetAsync(ctx->rblock, 0, kHandoverBytes + 256, ctx->stream));
+    ctx->rdirty = true;   // until the kernel has handed over and cleared the block
+    void* mapped = nullptr;
+    TGP_CUDA(cudaHostGetDevicePointer(&mapped, ctx->rhost, 0));
+    out->host = static_cast<unsigned long long*>(mapped);
+    out->block = ctx->rblock;
+    out->words16 = static_cast<uint32_t>((words + 1) / 2);
+    out->ticket = reinterpret_cast<uint32_t*>(ctx->rblock + kHandoverBytes / 8);
+    out->seq = ++ctx->rseq ? ctx->rseq : ++ctx->rseq;   // 0 is never a sequence number
+    ctx->rhost[2ull * out->words16] = 0;
+    return TGP_OK;
+}
+
+// Waits for the launch's handover: polls the sequence word for a while (the
+// poll sees it sooner than a stream synchronisation returns), then waits for
+// the stream, which also reports a failed launch.
+int handover_wait(tgp_ctx* ctx, const ResultOut& out) {
+    const volatile unsigned long long* flag = ctx->rhost + 2ull * out.words16;
+    const auto t0 = std::chrono::steady_clock::now();
+    for (uint32_t i = 1; *flag != out.seq; ++i) {
+        __builtin_ia32_pause();
+        if ((i & 255u) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
+            const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+            if (e != cudaSuccess || *flag != out.seq)
+                return fail(ctx, TGP_DEVICE_ERROR,
+                            std::string("result handover: ") + (e != cudaSuccess ? cudaGetErrorString(e) : "not written"));
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    ctx->rdirty = false;
     return TGP_OK;
 }
 
@@ -912,6 +970,7 @@ int try_launch_q1(tgp_ctx* ctx, const Plan& P, uint32_t mode, bool acc128, uint6
     A.nrows = P.nrows;
     A.acc = P.acc;
     A.counters = P.counters;
+    A.out = P.out;
     const uint64_t chunks = P.nrows / 128;
     const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((chunks + 15) / 16, static_cast<uint64_t>(ctx->sms) * 2));
     // A thread adds at most ceil(chunks / warps) chunks of four rows and four
@@ -1082,6 +1141,8 @@ int tgp_shutdown(tgp_ctx* ctx) {
     if (ctx->arena.base) cudaFree(ctx->arena.base);
     if (ctx->kin) cudaFree(ctx->kin);
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
+    if (ctx->rblock) cudaFree(ctx->rblock);
+    if (ctx->rhost) cudaFreeHost(ctx->rhost);
     for (auto& p : ctx->prof_events) {
         cudaEventDestroy(p.first);
         cudaEventDestroy(p.second);
@@ -2266,7 +2327,12 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     // One result block [counters: 4 words][error word: 2 words][accumulators],
     // cleared with one memset and read back with one copy.
     const uint64_t block_words = qs.block_words();
-    unsigned long long* block = cv.take<unsigned long long>(block_words);
+    ResultOut handover;
+    std::memset(&handover, 0, sizeof(handover));
+    if (mode != MODE_GROUP_HASH && !device_fmt && !(tn && ngroups_direct >= kDeviceFormatGroups) && P.nrows)
+        TGP_TRY(handover_begin(ctx, block_words, &handover));
+    unsigned long long* block = handover.host ? handover.block : cv.take<unsigned long long>(block_words);
+    P.out = handover;
     P.counters = block;
     P.err = reinterpret_cast<uint32_t*>(block + 4);
     P.acc = acc_words ? block + 6 : cv.take<unsigned long long>(2);
@@ -2274,7 +2340,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     uint8_t* fmt = device_fmt ? cv.take<uint8_t>(fmt_scratch) : nullptr;
     if (acc_words && qs.has_minmax()) {
         // Every group's accumulators from one image, written on the device.
-        TGP_CUDA(cudaMemsetAsync(block, 0, 48, ctx->stream));
+        if (!handover.host) TGP_CUDA(cudaMemsetAsync(block, 0, 48, ctx->stream));
         std::vector<unsigned long long> one;
         init_acc_image(P, 1, &one);
         SlotImage img;
@@ -2282,7 +2348,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         img.stride = nv1 * 2;
         std::copy(one.begin(), one.end(), img.w);
         TGP_CUDA(launch_fill_slots(P.acc, ngroups_direct, img, ctx->sms, ctx->stream));
-    } else {
+    } else if (!handover.host) {
         TGP_CUDA(cudaMemsetAsync(block, 0, block_words * 8, ctx->stream));
     }
     if (mode == MODE_GROUP_HASH && P.hpack && P.hdirect) {
@@ -2420,10 +2486,16 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         return TGP_OK;
     }
 
-    TGP_TRY(pinned_reserve(ctx, back_words * 8));
-    TGP_CUDA(cudaMemcpyAsync(ctx->hpin, block, back_words * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
-    const unsigned long long* hb = reinterpret_cast<const unsigned long long*>(ctx->hpin);
+    const unsigned long long* hb;
+    if (handover.host) {
+        TGP_TRY(handover_wait(ctx, handover));
+        hb = ctx->rhost;
+    } else {
+        TGP_TRY(pinned_reserve(ctx, back_words * 8));
+        TGP_CUDA(cudaMemcpyAsync(ctx->hpin, block, back_words * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        TGP_CUDA(cudaStreamSynchronize(ctx->stream));
+        hb = reinterpret_cast<const unsigned long long*>(ctx->hpin);
+    }
     unsigned long long counters[4] = {hb[0], hb[1], hb[2], hb[3]};
     const uint32_t err = static_cast<uint32_t>(hb[4] & 0xffffffffull);
     if (shrunk && (err & kErrHashFull) && !(err & kErrWaitTimeout))

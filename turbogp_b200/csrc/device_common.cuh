@@ -220,4 +220,33 @@ __device__ __forceinline__ int64_t add_wrap_checked(int64_t a, int64_t b, uint32
     return r;
 }
 
+// ---------------------------------------------------------------------------
+// End of a launch that hands its result to the host itself (ResultOut): called
+// by `nt` threads of every CTA (t = 0 .. nt - 1) after their last update of the
+// result block; `bar` is a barrier over those threads.
+// ---------------------------------------------------------------------------
+template <typename BAR>
+__device__ __forceinline__ void finish_result(const ResultOut& O, uint32_t t, uint32_t nt, BAR&& bar) {
+    if (!O.host) return;
+    __shared__ uint32_t last;
+    __threadfence();   // this thread's updates are performed before its CTA counts as done
+    bar();
+    if (t == 0) last = atomicAdd(O.ticket, 1u) == gridDim.x - 1u ? 1u : 0u;
+    bar();
+    if (!last) return;
+    __threadfence();
+    ulonglong2* blk = reinterpret_cast<ulonglong2*>(O.block);
+    ulonglong2* dst = reinterpret_cast<ulonglong2*>(O.host);
+    for (uint32_t i = t; i < O.words16; i += nt) {
+        dst[i] = __ldcg(blk + i);
+        blk[i] = make_ulonglong2(0ull, 0ull);
+    }
+    __threadfence_system();
+    bar();
+    if (t == 0) {
+        *O.ticket = 0;
+        *reinterpret_cast<volatile unsigned long long*>(O.host + 2ull * O.words16) = O.seq;
+    }
+}
+
 }  // namespace tgp

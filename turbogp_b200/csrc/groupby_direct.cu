@@ -636,6 +636,7 @@ __global__ void __launch_bounds__(kDgThreads, 2) q1_group_kernel(const Q1Args A)
             if (v == 0) atomicAdd(A.counters, sum);  // selected rows
         }
     }
+    finish_result(A.out, t, NT, [] { __syncthreads(); });
 }
 
 }  // namespace

@@ -181,6 +181,19 @@ struct alignas(16) RegBlock {
     int64_t vals_add[2][2];
 };
 
+// How a single launch hands its result block to the host (finish_result): the
+// last CTA to finish copies the block's 16-byte words into mapped page-locked
+// memory, leaves the block zero for the next query and then stores `seq`
+// behind the copy. No clear before the kernel, no copy and no stream
+// synchronisation after it. host = null: the host clears and copies.
+struct ResultOut {
+    unsigned long long* host;   // mapped: [words16 * 2 words][seq]
+    unsigned long long* block;  // device, 16-byte aligned
+    uint32_t words16;
+    uint32_t seq;
+    uint32_t* ticket;           // CTAs done (0 at rest)
+};
+
 struct alignas(16) Plan {
     uint64_t nrows;
     uint32_t nslots;
@@ -286,6 +299,7 @@ struct alignas(16) Plan {
     uint32_t hpack_shift;
     int64_t hpack_bias;
     uint32_t jpay_w;
+    ResultOut out;
     uint32_t two_ctas;      // launch the register budget of two CTAs per SM (join-payload limb-table shapes)
     RegBlock rb;                    // filled by fill_reg_block before every launch
 };

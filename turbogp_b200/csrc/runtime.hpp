@@ -63,6 +63,7 @@ struct Q1Args {
     uint64_t nrows;
     unsigned long long* acc;
     unsigned long long* counters;
+    ResultOut out;
 };
 // GROUP BY one sparse key into 16-byte hash slots [key][count << shift + sum]
 // under at most four int32 leaves (groupby_direct.cu). hs: keep the per-CTA
@@ -336,6 +337,13 @@ struct tgp_ctx {
     // Pinned host staging for small readbacks.
     uint8_t* hpin = nullptr;
     size_t hpin_cap = 0;
+    // Result blocks handed over by the kernel (ResultOut): a device block that
+    // is zero between queries, its ticket, and the mapped host copy with the
+    // sequence word. Null until the first query that fits.
+    unsigned long long* rblock = nullptr;
+    unsigned long long* rhost = nullptr;
+    uint32_t rseq = 0;
+    bool rdirty = false;   // not handed over since its last use: clear the block first
     // Device staging of kernel-table inputs (kept apart from the arena so
     // scans that grow the arena never move a staged input).
     uint8_t* kin = nullptr;

@@ -2201,15 +2201,21 @@ __global__ void __launch_bounds__(NT + 32, MINB) scan_kernel(const __grid_consta
     __syncthreads();
     PipeState st;
     if (t >= static_cast<uint32_t>(NT)) {
-        if (t != static_cast<uint32_t>(NT)) return;
-        pipe_produce(P, full, empty, stages, blockIdx.x, G, count, st, &abort_flag);
-        // Drain: the last min(S, n) copies have landed before this thread
-        // exits (earlier ones were waited for through empty[]).
-        const uint32_t S = P.nstages;
-        const uint64_t first = st.n > S ? st.n - S : 0;
-        for (uint64_t i = first; i < st.n; ++i)
-            if (!mbar_wait_bounded(&full[i % S], static_cast<uint32_t>((i / S) & 1u), P.wait_ns))
-                atomicOr(P.err, kErrWaitTimeout);
+        if (t == static_cast<uint32_t>(NT)) {
+            pipe_produce(P, full, empty, stages, blockIdx.x, G, count, st, &abort_flag);
+            // Drain: the last min(S, n) copies have landed before this thread
+            // exits (earlier ones were waited for through empty[]).
+            const uint32_t S = P.nstages;
+            const uint64_t first = st.n > S ? st.n - S : 0;
+            for (uint64_t i = first; i < st.n; ++i)
+                if (!mbar_wait_bounded(&full[i % S], static_cast<uint32_t>((i / S) & 1u), P.wait_ns))
+                    atomicOr(P.err, kErrWaitTimeout);
+        }
+        // The result is handed over only after this warp's last error bit.
+        if (P.out.host) {
+            __syncwarp();
+            asm volatile("bar.arrive 2, %0;" ::"n"(NT + 32) : "memory");
+        }
         return;
     }
     RegLeaves RL;
@@ -2222,6 +2228,10 @@ __global__ void __launch_bounds__(NT + 32, MINB) scan_kernel(const __grid_consta
     // Every consumer reaches the flush, also after a timeout (the host then
     // discards the result), so the consumer barrier inside it always completes.
     sink.flush(P, extra, t);
+    if (P.out.host) {
+        asm volatile("bar.sync 2, %0;" ::"n"(NT + 32) : "memory");
+        finish_result(P.out, t, static_cast<uint32_t>(NT), [] { consumer_sync<NT>(); });
+    }
 }
 
 // ---------------------------------------------------------------------------
