@@ -27,6 +27,14 @@ constexpr uint64_t kDirectMaxGroups = 1ull << 22;
 constexpr uint64_t kHashDirectMax = 1ull << 27;   // key values of a directly indexed group table
 constexpr uint64_t kDeviceFormatGroups = 4096;         // direct groups formatted on the device from here on
 constexpr size_t kStagedResultBytes = 4u << 20;        // formatted results that come back through ctx->hpin
+// Join payloads the streaming probe keeps in a CTA's shared memory: the bytes
+// themselves, or one match bit each.
+constexpr uint64_t kPayBytesMax = 160u << 10, kPayBitsMax = (190ull << 10) * 8;
+constexpr size_t kPayBitsSmem = 195u << 10;   // shared memory of the bits form (its L1 serves the payload bytes)
+inline bool pay_bytes_fit(uint64_t entries) { return entries <= kPayBytesMax; }
+inline bool pay_bits_fit(uint64_t entries, uint32_t width) {
+    return width == 1 && !pay_bytes_fit(entries) && entries <= kPayBitsMax;
+}
 constexpr size_t kJoinSmemCap = 144u << 10;        // shared memory per CTA of a payload-join scan (see size_smem)
 
 int fail(tgp_ctx* ctx, int st, const std::string& m) {
@@ -929,7 +937,7 @@ int try_launch_q1(tgp_ctx* ctx, const Plan& P, uint32_t mode, bool acc128, uint6
     // An armed failure-path hook (tgp_debug_fail_next_scan) targets the scan
     // pipeline's stage copies; this kernel has no stage ring and no waits.
     if (ctx->dbg_skip_tile1) return TGP_OK;
-    if (mode != MODE_GROUP_PRIVATE || acc128 || P.shape != 1 || !P.dense_vec || P.jslot >= 0 || P.ngkey != 2 ||
+    if (mode != MODE_GROUP_PRIVATE || acc128 || P.shape != kShapeQ1 || !P.dense_vec || P.jslot >= 0 || P.ngkey != 2 ||
         !P.sum64 || P.check_ovf || P.nval != 4 || P.chain.nsteps != 4 || ngroups == 0 || ngroups > 0xffffffffull)
         return TGP_OK;
     if (P.nleaf > 4 || (P.nleaf && !(P.all_and && P.kend[0] == P.nleaf))) return TGP_OK;
@@ -987,6 +995,70 @@ int try_launch_q1(tgp_ctx* ctx, const Plan& P, uint32_t mode, bool acc128, uint6
     return TGP_OK;
 }
 
+// The join shape on a payload array (MODE_GROUP_SHARED32, groups from the build
+// side, at most four int32 leaves): the streaming probe of join_stream.cu when
+// the payload bytes or the match bits fit a CTA's shared memory (else false,
+// nothing launched). A table is loaded once per CTA: from a row per 16 bytes of
+// it on the load is repaid (2M rows x 1.5M keys, 13.5K rows per CTA: 49 -> 33
+// us); fewer rows stay with the scan engine.
+int try_launch_join(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroups, bool* done) {
+    *done = false;
+    if (ctx->dbg_skip_tile1 || mode != MODE_GROUP_SHARED32 || P.shape != kShapeJoin || !P.dense_vec || !P.jpay ||
+        P.jpay_w != 1 || !P.sum64 || P.check_ovf || P.nval != 1 || P.chain.nsteps != 2 || ngroups == 0 || ngroups > 254 ||
+        P.jslot < 0 || P.slot[P.jslot].dtype != DT_I32 || P.jkrange >= 0xffffffffull)
+        return TGP_OK;
+    if (P.nleaf > 4 || (P.nleaf && !(P.all_and && P.kend[0] == P.nleaf))) return TGP_OK;
+    for (uint32_t k = 0; k < P.ngkey; ++k)
+        if (!P.gkey[k].build_side || P.gkey[k].lut) return TGP_OK;
+    const uint64_t entries = P.jkrange + 1;
+    const bool bytes = pay_bytes_fit(entries);
+    const size_t budget = bytes ? ctx->max_dyn_smem - 1024 : kPayBitsSmem;
+    if (!bytes && !P.jbits) return TGP_OK;
+    JoinStreamArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.table = bytes ? static_cast<const void*>(P.jpay) : static_cast<const void*>(P.jbits);
+    A.table_bytes = static_cast<uint32_t>(bytes ? (entries + 15) & ~uint64_t{15} : pay_bits_words(entries) * 4);
+    A.ngroups = static_cast<uint32_t>(ngroups);
+    A.copies = 32;   // one per warp
+    while (A.copies > 1 && join_stream_smem(A.table_bytes, A.copies, A.ngroups) > budget) A.copies >>= 1;
+    if (join_stream_smem(A.table_bytes, A.copies, A.ngroups) > budget) return TGP_OK;
+    const uint64_t chunks = (P.nrows + 127) / 128;
+    const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((chunks + 31) / 32, static_cast<uint64_t>(ctx->sms)));
+    if (P.nrows / grid < A.table_bytes / 16) return TGP_OK;
+    auto slot_ptr = [&](uint32_t soff) -> const uint8_t* {
+        for (uint32_t k = 0; k < P.nslots; ++k)
+            if (P.slot[k].smem_off == soff) return P.slot[k].ptr;
+        return nullptr;
+    };
+    for (uint32_t i = 0; i < P.nleaf; ++i) {
+        A.leaf_col[i] = P.slot[P.leaf[i].slot].ptr;
+        A.leaf_lo[i] = P.leaf[i].lo32;
+        A.leaf_sp[i] = P.leaf[i].span32;
+        if (P.leaf[i].negate) A.leaf_neg |= 1u << i;
+    }
+    A.nleaf = P.nleaf;
+    A.key = P.slot[P.jslot].ptr;
+    A.col0 = slot_ptr(P.chain.s[0].soff);
+    A.col1 = slot_ptr(P.chain.s[1].soff);
+    if (!A.col0 || !A.col1 || P.chain.s[1].acc != 1) return TGP_OK;
+    A.mul = static_cast<uint32_t>(P.chain.s[1].mul32);
+    A.add = static_cast<uint32_t>(P.chain.s[1].add32);
+    A.kmin = static_cast<uint32_t>(P.jkmin);
+    A.krange = static_cast<uint32_t>(P.jkrange);
+    A.pay = reinterpret_cast<const uint8_t*>(P.jpay);
+    A.nrows = P.nrows;
+    A.acc = P.acc;
+    A.counters = P.counters;
+    A.out = P.out;
+    std::pair<cudaEvent_t, cudaEvent_t>* ev = nullptr;
+    TGP_TRY(profile_begin(ctx, &ev));
+    const cudaError_t e = launch_join_stream(A, !bytes, static_cast<int>(grid), ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("join launch: ") + cudaGetErrorString(e));
+    if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
+    *done = true;
+    return TGP_OK;
+}
+
 int get_table(tgp_ctx* ctx, tgp_table_id id, const Table** out) {
     auto it = ctx->tables.find(id);
     if (it == ctx->tables.end()) return fail(ctx, TGP_NOT_FOUND, "unknown table id");
@@ -1027,7 +1099,10 @@ int upload(tgp_ctx* ctx, void* dst, const void* src, size_t bytes) {
 void free_join(tgp_ctx* ctx, JoinTable& J) {
     dev_free(ctx, J.tab);
     J.tab = nullptr;
-    for (auto& kv : J.pays) dev_free(ctx, kv.second.ptr);
+    for (auto& kv : J.pays) {
+        dev_free(ctx, kv.second.ptr);
+        dev_free(ctx, kv.second.bits);
+    }
     J.pays.clear();
 }
 
@@ -2017,22 +2092,36 @@ static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t s
         if (dry) {
             // Sizing only (tgp_query_footprint): a payload still to be built
             // counts as memory the query needs; nothing is launched.
-            if (pt == J->pays.end()) qs.pending_dev_bytes += entries * pw;
+            if (pt == J->pays.end()) qs.pending_dev_bytes += entries * pw + (pay_bits_fit(entries, pw) ? pay_bits_words(entries) * 4 : 0);
             P.jpay = pt != J->pays.end() ? pt->second.ptr : (J->pays.empty() ? nullptr : J->pays.begin()->second.ptr);
         } else {
             if (pt == J->pays.end()) {
                 JoinTable::Payload np;
                 np.width = pw;
-                TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&np.ptr), std::max<uint64_t>(entries * pw, 16),
+                TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&np.ptr), ((entries * pw + 15) & ~uint64_t{15}),   // read in 16-byte words
                                   "join payload allocation failed"));
                 const cudaError_t e = launch_join_pay(J->tab, J->cap, K, np.ptr, pw, entries, ctx->sms, ctx->stream);
                 if (e != cudaSuccess) {
                     dev_free(ctx, np.ptr);
                     return fail(ctx, TGP_DEVICE_ERROR, std::string("join payload: ") + cudaGetErrorString(e));
                 }
+                // Keys whose match bits fit a CTA's shared memory, but whose
+                // payload bytes do not: the streaming probe's table.
+                if (pay_bits_fit(entries, pw) &&
+                    dev_alloc(ctx, reinterpret_cast<void**>(&np.bits), pay_bits_words(entries) * 4,
+                              "join match bits allocation failed") == TGP_OK) {
+                    const cudaError_t be =
+                        launch_pay_bits(reinterpret_cast<const uint8_t*>(np.ptr), entries, np.bits, ctx->sms, ctx->stream);
+                    if (be != cudaSuccess) {
+                        dev_free(ctx, np.ptr);
+                        dev_free(ctx, np.bits);
+                        return fail(ctx, TGP_DEVICE_ERROR, std::string("join match bits: ") + cudaGetErrorString(be));
+                    }
+                }
                 pt = J->pays.emplace(sig, np).first;
             }
             P.jpay = pt->second.ptr;
+            P.jbits = pt->second.bits;
         }
         qs.pay_sig = sig;
         P.jpay_w = pw;
@@ -2377,6 +2466,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     } else {
         bool done = false;
         TGP_TRY(try_launch_q1(ctx, P, mode, acc128, ngroups_direct, b.max_abs_val, &done));
+        if (!done) TGP_TRY(try_launch_join(ctx, P, mode, ngroups_direct, &done));
         if (!done) TGP_TRY(launch(ctx, P, mode, acc128));
     }
 
@@ -3772,6 +3862,7 @@ int tgp_batch_submit(tgp_ctx* ctx, tgp_batch_item* items, uint32_t n, tgp_batch_
         const QueryState& qs = B->qs[i];
         bool done = false;
         TGP_TRY(try_launch_q1(ctx, qs.b->P, qs.mode, qs.acc128, qs.ngroups_direct, qs.b->max_abs_val, &done));
+        if (!done) TGP_TRY(try_launch_join(ctx, qs.b->P, qs.mode, qs.ngroups_direct, &done));
         if (!done) TGP_TRY(launch(ctx, qs.b->P, qs.mode, qs.acc128));
     }
     for (auto& M : B->merges) {

@@ -88,6 +88,8 @@ struct Leaf {
 
 // Plan::shape of scalar aggregates on the register fast path.
 constexpr uint32_t kShapeScalar = 0xffffu;
+// The fixed value programs, in the order of the scan engine's shape table.
+constexpr uint32_t kShapeQ1 = 1, kShapeJoin = 2;
 
 // Postfix program opcodes: values < kMaxLeaves push leaf i.
 enum : uint8_t { OP_AND = 0x80, OP_OR = 0x81, OP_NOT = 0x82 };
@@ -299,6 +301,7 @@ struct alignas(16) Plan {
     uint32_t hpack_shift;
     int64_t hpack_bias;
     uint32_t jpay_w;
+    const uint32_t* jbits;  // one bit per payload entry (a build row matches), or null
     ResultOut out;
     uint32_t two_ctas;      // launch the register budget of two CTAs per SM (join-payload limb-table shapes)
     RegBlock rb;                    // filled by fill_reg_block before every launch

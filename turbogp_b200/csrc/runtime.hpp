@@ -88,6 +88,33 @@ struct HashGroupArgs {
     uint32_t* err;
     unsigned long long* counters;  // [0] += selected rows
 };
+// Streaming join probe with grouped aggregation (join_stream.cu): int32 probe
+// keys, u8 payload entries, sum(col0 * (mul * col1 + add)) and COUNT(*) per
+// payload group, accumulators [g][2][2] (int64 sums in their low limbs).
+struct JoinStreamArgs {
+    const uint8_t* leaf_col[4];
+    uint32_t leaf_lo[4], leaf_sp[4];
+    uint32_t leaf_neg, nleaf;
+    const uint8_t* key;
+    const uint8_t* col0;           // int64
+    const uint8_t* col1;           // int32
+    uint32_t mul, add;             // mul * col1 + add is never negative
+    uint32_t kmin, krange;
+    const uint8_t* pay;            // payload bytes in global memory
+    const void* table;             // what a CTA keeps in shared memory: the payload bytes or the match bits,
+    uint32_t table_bytes;          // whole 16-byte words
+    uint32_t ngroups, copies;      // limb tables (a power of two)
+    uint64_t nrows;
+    unsigned long long* acc;
+    unsigned long long* counters;
+    ResultOut out;
+};
+inline size_t join_stream_smem(uint32_t table_bytes, uint32_t copies, uint32_t ngroups) {
+    return table_bytes + static_cast<size_t>(copies) * ngroups * 12;
+}
+uint64_t pay_bits_words(uint64_t entries);
+cudaError_t launch_pay_bits(const uint8_t* pay, uint64_t entries, uint32_t* bits, int sms, cudaStream_t st);
+cudaError_t launch_join_stream(const JoinStreamArgs& A, bool bits, int grid, cudaStream_t st);
 bool hash_group_supported(uint32_t kdt, uint32_t vdt);
 uint64_t hash_group_grid(uint64_t nrows, int sms);
 uint64_t hash_group_rows_per_cta(uint64_t nrows, int sms);
@@ -281,6 +308,7 @@ struct JoinTable {
     struct Payload {
         uint32_t* ptr = nullptr;
         uint32_t width = 4;
+        uint32_t* bits = nullptr;   // one bit per entry (a build row matches), or null
     };
     std::map<std::vector<uint64_t>, Payload> pays;
 };

@@ -2489,7 +2489,7 @@ static ShapeEntry shape_entry() {
 }
 
 static const ShapeEntry* shape_table(uint32_t* n) {
-    static const ShapeEntry table[] = {shape_entry<ShapeQ1>(), shape_entry<ShapeJoin>()};
+    static const ShapeEntry table[] = {shape_entry<ShapeQ1>(), shape_entry<ShapeJoin>()};   // kShapeQ1, kShapeJoin
     *n = sizeof(table) / sizeof(table[0]);
     return table;
 }
