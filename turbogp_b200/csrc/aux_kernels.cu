@@ -638,6 +638,47 @@ __global__ void __launch_bounds__(kAuxThreads) format_direct_kernel(const unsign
     }
 }
 
+// Tables of at most kDirOneSlots slots in one pass: every block counts the
+// occupied slots before its own 256 itself (a few coalesced reads of a table
+// that lies in L2), so there is no scan and the host does not have to learn the
+// number of groups before the groups are written. *total = that number.
+__global__ void __launch_bounds__(kAuxThreads) format_direct_one_kernel(const unsigned long long* htab, uint64_t nslots,
+                                                                        const HashFormat F, uint64_t* keys_out,
+                                                                        tgp_agg_value* vals_out,
+                                                                        unsigned long long* total) {
+    __shared__ uint32_t wsum[kAuxThreads / 32], wocc[kAuxThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, cw = count_word(F);
+    const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kAuxThreads;
+    uint32_t before = 0;
+#pragma unroll 4
+    for (uint64_t i = threadIdx.x; i < base; i += kAuxThreads) before += htab[i * F.hstride + cw] != 0ull ? 1u : 0u;
+    before = __reduce_add_sync(0xffffffffu, before);
+    const uint64_t i = base + threadIdx.x;
+    const unsigned long long* s = htab + i * F.hstride;
+    const bool occ = i < nslots && s[cw] != 0ull;
+    const uint32_t mask = __ballot_sync(0xffffffffu, occ);
+    if (lane == 0) {
+        wsum[warp] = before;
+        wocc[warp] = __popc(mask);
+    }
+    __syncthreads();
+    uint32_t pos = __popc(mask & ((1u << lane) - 1u)), all = 0;
+    for (uint32_t w = 0; w < kAuxThreads / 32; ++w) {
+        pos += wsum[w] + (w < warp ? wocc[w] : 0u);
+        all += wsum[w] + wocc[w];
+    }
+    if (occ) write_group(s, i, pos, F, keys_out, vals_out);
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) *total = all;
+}
+
+cudaError_t format_direct_one(const unsigned long long* htab, uint64_t nslots, const HashFormat& F, uint64_t* keys_out,
+                              tgp_agg_value* vals_out, unsigned long long* total, cudaStream_t st) {
+    if (nslots == 0) return cudaMemsetAsync(total, 0, 8, st);
+    format_direct_one_kernel<<<static_cast<unsigned>((nslots + kAuxThreads - 1) / kAuxThreads), kAuxThreads, 0, st>>>(
+        htab, nslots, F, keys_out, vals_out, total);
+    return cudaGetLastError();
+}
+
 cudaError_t format_hash_groups(const unsigned long long* packed, uint64_t n, const HashFormat& F, uint32_t key_bits,
                                void* scratch, size_t scratch_bytes, uint64_t* keys_out, tgp_agg_value* vals_out,
                                int sms, cudaStream_t st) {

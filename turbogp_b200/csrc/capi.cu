@@ -26,6 +26,7 @@ constexpr unsigned long long kEmptySlot = ~0ull;
 constexpr uint64_t kDirectMaxGroups = 1ull << 22;
 constexpr uint64_t kHashDirectMax = 1ull << 27;   // key values of a directly indexed group table
 constexpr uint64_t kDeviceFormatGroups = 4096;         // direct groups formatted on the device from here on
+constexpr size_t kOnePassBytes = 1536u << 10;          // results formatted with room for every slot (30 us of link)
 constexpr size_t kStagedResultBytes = 4u << 20;        // formatted results that come back through ctx->hpin
 // Join payloads the streaming probe keeps in a CTA's shared memory: the bytes
 // themselves, or one match bit each.
@@ -2410,7 +2411,12 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     const uint64_t htab_words = hcap * P.hstride;
     const bool device_fmt = !tn && formats_direct(qs, q);
     const uint64_t fmt_slots = mode == MODE_GROUP_HASH ? hcap : ngroups_direct;
-    const size_t fmt_scratch = device_fmt ? direct_groups_scratch(fmt_slots) : 0;
+    // Moderate tables are formatted in one pass, with room for every slot, and
+    // come back with the counters; larger ones are counted first.
+    const size_t one_keys = keys_out ? (fmt_slots * q->ngroup * 8 + 255) & ~size_t{255} : 0;
+    const size_t one_bytes = one_keys + (vals_out ? fmt_slots * q->nagg * sizeof(tgp_agg_value) : 0);
+    const bool one_pass = device_fmt && fmt_slots <= kDirOneSlots && one_bytes <= kOnePassBytes;
+    const size_t fmt_scratch = one_pass ? one_bytes : device_fmt ? direct_groups_scratch(fmt_slots) : 0;
     Carve cv;
     TGP_TRY(arena_reserve(ctx, acc_words * 8 + htab_words * 8 + fmt_scratch + 2048, &cv));
     // One result block [counters: 4 words][error word: 2 words][accumulators],
@@ -2506,7 +2512,12 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     uint64_t back_words = block_words;
     if (device_fmt) {
         back_words = 6;
-        TGP_CUDA(count_direct_groups(table, fmt_slots, group_format(), fmt, fmt_scratch, P.counters + 2, ctx->stream));
+        if (one_pass)
+            TGP_CUDA(format_direct_one(table, fmt_slots, group_format(), keys_out ? reinterpret_cast<uint64_t*>(fmt) : nullptr,
+                                       vals_out ? reinterpret_cast<tgp_agg_value*>(fmt + one_keys) : nullptr, P.counters + 2,
+                                       ctx->stream));
+        else
+            TGP_CUDA(count_direct_groups(table, fmt_slots, group_format(), fmt, fmt_scratch, P.counters + 2, ctx->stream));
     }
 
     // Top-N of many groups by selection: the groups are listed and narrowed
@@ -2581,7 +2592,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         TGP_TRY(handover_wait(ctx, handover));
         hb = ctx->rhost;
     } else {
-        TGP_TRY(pinned_reserve(ctx, back_words * 8));
+        TGP_TRY(pinned_reserve(ctx, back_words * 8 + 256 + (one_pass ? one_bytes : 0)));
         TGP_CUDA(cudaMemcpyAsync(ctx->hpin, block, back_words * 8, cudaMemcpyDeviceToHost, ctx->stream));
         TGP_CUDA(cudaStreamSynchronize(ctx->stream));
         hb = reinterpret_cast<const unsigned long long*>(ctx->hpin);
@@ -2739,6 +2750,8 @@ int tgp_query_footprint(tgp_ctx* ctx, const tgp_query* q, uint64_t* device_bytes
     if (!ctx || !q || !device_bytes) return fail(ctx, TGP_INVALID_ARG, "null argument");
     QueryState qs;
     TGP_TRY(plan_query(ctx, q, qs, scan_kernel_static_smem(), nullptr, /*dry=*/true));
+        if (one_pass && one_bytes)
+            TGP_CUDA(cudaMemcpyAsync(ctx->hpin + 256, fmt, one_bytes, cudaMemcpyDeviceToHost, ctx->stream));
     plan_one_word_slots(qs, q, nullptr);
     const Plan& P = qs.b->P;
     // What execute_impl carves or allocates for one run of the query.
@@ -2756,6 +2769,11 @@ int tgp_query_footprint(tgp_ctx* ctx, const tgp_query* q, uint64_t* device_bytes
         }
         bytes += max_groups * (8ull * q->ngroup + sizeof(tgp_agg_value) * q->nagg) + 512;  // formatted result
     } else if (formats_direct(qs, q)) {
+        if (one_pass) {
+            if (keys_out) std::memcpy(keys_out, ctx->hpin + 256, ng * q->ngroup * 8);
+            if (vals_out) std::memcpy(vals_out, ctx->hpin + 256 + one_keys, ng * nagg * sizeof(tgp_agg_value));
+            return TGP_OK;
+        }
         bytes += direct_groups_scratch(qs.ngroups_direct) +
                  qs.ngroups_direct * (8ull * q->ngroup + sizeof(tgp_agg_value) * q->nagg) + 512;
     }

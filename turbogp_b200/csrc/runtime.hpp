@@ -258,6 +258,11 @@ cudaError_t top_select_narrow(const unsigned long long* htab, uint64_t max_group
 cudaError_t launch_delay(uint64_t ns, cudaStream_t st);
 // Device-to-host copy by a kernel into page-locked (mapped) host memory; both
 // addresses and the size 16-byte aligned.
+// The same in one pass over a table of at most kDirOneSlots slots; the outputs
+// have room for every slot.
+constexpr uint64_t kDirOneSlots = 32768;
+cudaError_t format_direct_one(const unsigned long long* htab, uint64_t nslots, const HashFormat& F, uint64_t* keys_out,
+                              tgp_agg_value* vals_out, unsigned long long* total, cudaStream_t st);
 cudaError_t launch_copy_to_host(void* host_dst, const void* dev_src, size_t bytes, cudaStream_t st);
 cudaError_t launch_like(const uint8_t* bytes, const unsigned long long* offs, uint64_t n, const LikePattern& P,
                         bool negated, uint32_t* bitmap, unsigned long long* count, uint32_t* err, int sms,
