@@ -13,7 +13,7 @@ use std::env;
 use std::path::{Path, PathBuf};
 use std::process::Command;
 
-const SOURCES: [&str; 8] = ["scan_engine.cu", "aux_kernels.cu", "groupby_direct.cu", "join_pairs.cu", "group_select.cu", "join_stream.cu", "capi.cu", "noalloc.cu"];
+const SOURCES: [&str; 9] = ["scan_engine.cu", "aux_kernels.cu", "groupby_direct.cu", "join_pairs.cu", "group_select.cu", "join_stream.cu", "group_stream.cu", "capi.cu", "noalloc.cu"];
 
 fn nvcc() -> PathBuf {
     if let Ok(p) = env::var("NVCC") {

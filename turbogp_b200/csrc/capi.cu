@@ -1060,6 +1060,163 @@ int try_launch_join(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroups
     return TGP_OK;
 }
 
+// A limb-table plan (MODE_GROUP_SHARED32) whose keys and leaves are int32 or
+// u8 columns and whose values are sums, counts or extremes of single columns
+// or one of the fixed programs: the streaming kernel of group_stream.cu (else
+// false, nothing launched).
+int try_launch_group(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroups, bool* done) {
+    *done = false;
+    if (ctx->dbg_skip_tile1 || mode != MODE_GROUP_SHARED32 || !P.sum64 || P.check_ovf || P.nrows == 0 || ngroups == 0)
+        return TGP_OK;
+    if (P.nleaf > 4 || (P.nleaf && !(P.all_and && P.kend[0] == P.nleaf))) return TGP_OK;
+    GroupStreamArgs A;
+    std::memset(&A, 0, sizeof(A));
+    A.nrows = P.nrows;
+    for (uint32_t i = 0; i < P.nleaf; ++i) {
+        A.leaf_col[i] = P.slot[P.leaf[i].slot].ptr;
+        A.leaf_lo[i] = P.leaf[i].lo32;
+        A.leaf_sp[i] = P.leaf[i].span32;
+        if (P.leaf[i].negate) A.leaf_neg |= 1u << i;
+    }
+    A.nleaf = P.nleaf;
+    uint32_t off = 0;   // shared memory taken so far
+    int pay = GS_PAY_NONE;
+    if (P.jslot >= 0) {
+        if (!P.jpay || P.jpay_w != 1 || P.slot[P.jslot].dtype != DT_I32 || P.jkrange >= 0xffffffffull) return TGP_OK;
+        const uint64_t entries = P.jkrange + 1;
+        const bool bytes = pay_bytes_fit(entries);
+        if (!bytes && !P.jbits) return TGP_OK;
+        pay = bytes ? GS_PAY_BYTES : GS_PAY_BITS;
+        A.table = bytes ? static_cast<const void*>(P.jpay) : static_cast<const void*>(P.jbits);
+        A.table_bytes = static_cast<uint32_t>(bytes ? (entries + 15) & ~uint64_t{15} : pay_bits_words(entries) * 4);
+        A.fk = P.slot[P.jslot].ptr;
+        A.pay = reinterpret_cast<const uint8_t*>(P.jpay);
+        A.kmin = static_cast<uint32_t>(P.jkmin);
+        A.krange = static_cast<uint32_t>(P.jkrange);
+        off = A.table_bytes;
+    }
+    auto slot_at = [&](uint32_t soff) -> const SlotDesc* {
+        for (uint32_t k = 0; k < P.nslots; ++k)
+            if (P.slot[k].smem_off == soff) return &P.slot[k];
+        return nullptr;
+    };
+    for (uint32_t k = 0; k < P.ngkey; ++k) {
+        const GKey& K = P.gkey[k];
+        if (K.build_side) {
+            if (K.lut) return TGP_OK;
+            continue;   // its part comes with the payload
+        }
+        if (K.slot < 0 || A.nkey == static_cast<uint32_t>(kGsKeys) || (K.dtype != DT_I32 && K.dtype != DT_U8)) return TGP_OK;
+        auto& G = A.key[A.nkey++];
+        G.col = P.slot[K.slot].ptr;
+        G.dtype = K.dtype;
+        G.min = static_cast<uint32_t>(K.min);
+        G.stride = static_cast<uint32_t>(K.stride);
+        if (K.lut) {
+            if (P.lut_cells[k] == 0 || P.lut_cells[k] > (8u << 10)) return TGP_OK;
+            G.lut = K.lut;
+            G.cells = P.lut_cells[k];
+            G.lut_off = off;
+            off += (G.cells + 15u) & ~15u;
+        }
+    }
+    // Values.
+    int vs = GS_COLS;
+    A.nval = P.nval;
+    for (uint32_t v = 0; v < P.nval; ++v) {
+        GroupStreamOp& O = A.op[v];
+        O.off = 4u * P.s32_off[v];
+        O.kind = P.s32_kind[v];
+        O.slot = v + 1;
+        O.ref64 = P.s32_ref[v];
+        O.ref = static_cast<uint32_t>(P.s32_ref[v]);
+    }
+    if (P.shape == kShapeQ1 || P.shape == kShapeJoin) {
+        vs = P.shape == kShapeQ1 ? GS_Q1 : GS_JOIN;
+        // The program's int64 column first, then its int32 ones in step order.
+        const int order[4] = {P.shape == kShapeQ1 ? 1 : 0, P.shape == kShapeQ1 ? 0 : 1, 2, 3};
+        const uint32_t n = P.shape == kShapeQ1 ? 4u : 2u;
+        if (P.chain.nsteps != n || P.nval != (P.shape == kShapeQ1 ? 4u : 1u)) return TGP_OK;
+        for (uint32_t i = 0; i < n; ++i) {
+            const ChainStep& S = P.chain.s[order[i]];
+            const SlotDesc* d = slot_at(S.soff);
+            if (!d) return TGP_OK;
+            A.col[i].col = d->ptr;
+            A.col[i].dtype = d->dtype;
+            if (i == 0) continue;
+            const uint32_t f = P.shape == kShapeQ1 ? i - 1 : 1u;   // factor index: q1 qty, disc, tax; join disc
+            A.mul[f] = static_cast<uint32_t>(S.mul32);
+            A.add[f] = static_cast<uint32_t>(S.add32);
+        }
+    } else {
+        // Values grouped by their column. (Products of two columns as well took
+        // the kernel past its 64 registers: 20M rows, 2,526 groups 0.175 ->
+        // 0.21 ms without a product among the values.)
+        int at[kMaxSlots];
+        std::fill(at, at + kMaxSlots, -1);
+        for (uint32_t v = 0; v < P.nval; ++v) {
+            const ValDesc& V = P.val[v];
+            const int s = V.nf == 1 ? V.f[0].slot : -1;
+            if (s < 0 || V.f[0].build_side || P.slot[s].dtype == DT_F64) return TGP_OK;
+            if (at[s] >= 0) continue;
+            if (A.ncol == static_cast<uint32_t>(kGsCols)) return TGP_OK;
+            at[s] = static_cast<int>(A.ncol);
+            A.col[A.ncol].col = P.slot[s].ptr;
+            A.col[A.ncol++].dtype = P.slot[s].dtype;
+        }
+        std::vector<GroupStreamOp> ops;
+        for (uint32_t c = 0; c < A.ncol; ++c) {
+            A.col[c].first = static_cast<uint32_t>(ops.size());
+            for (uint32_t v = 0; v < P.nval; ++v) {
+                const ValDesc& V = P.val[v];
+                if (at[V.f[0].slot] != static_cast<int>(c)) continue;
+                GroupStreamOp O = A.op[v];
+                O.mul = V.f[0].mul;
+                O.add = V.f[0].add;
+                O.ident = O.mul == 1 && O.add == 0;
+                O.nz = V.kind == VK_COUNT_NZ;
+                if (O.nz && O.kind != S32_NARROW) return TGP_OK;
+                ops.push_back(O);
+                ++A.col[c].nops;
+            }
+        }
+        std::copy(ops.begin(), ops.end(), A.op);
+    }
+    A.ngroups = static_cast<uint32_t>(ngroups);
+    A.words = P.s32_words;
+    A.acc_stride = P.nval + 1;
+    A.tab_off = off;
+    const size_t entry = static_cast<size_t>(ngroups) * P.s32_words * 4;
+    const size_t budget = pay == GS_PAY_BITS ? kPayBitsSmem : ctx->max_dyn_smem - 1024;
+    if (off + entry > budget) return TGP_OK;
+    A.copies = 32;
+    while (A.copies > 1 && off + A.copies * entry > budget) A.copies >>= 1;
+    const uint64_t chunks = (P.nrows + 127) / 128;
+    const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((chunks + 31) / 32, static_cast<uint64_t>(ctx->sms)));
+    // The tables are filled, cleared and merged once per CTA.
+    if (P.nrows / grid < (off + entry) / 16) return TGP_OK;
+    A.acc = P.acc;
+    A.counters = P.counters;
+    A.out = P.out;
+    std::pair<cudaEvent_t, cudaEvent_t>* ev = nullptr;
+    TGP_TRY(profile_begin(ctx, &ev));
+    const cudaError_t e = launch_group_stream(A, vs, pay, static_cast<uint32_t>(off + A.copies * entry), static_cast<int>(grid),
+                                              ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("group launch: ") + cudaGetErrorString(e));
+    if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
+    *done = true;
+    return TGP_OK;
+}
+
+// One query's launch: the streaming kernel its plan fits, else the scan engine.
+int launch_query(tgp_ctx* ctx, const Plan& P, uint32_t mode, bool acc128, uint64_t ngroups, uint64_t max_abs_val) {
+    bool done = false;
+    TGP_TRY(try_launch_q1(ctx, P, mode, acc128, ngroups, max_abs_val, &done));
+    if (!done) TGP_TRY(try_launch_join(ctx, P, mode, ngroups, &done));
+    if (!done) TGP_TRY(try_launch_group(ctx, P, mode, ngroups, &done));
+    return done ? TGP_OK : launch(ctx, P, mode, acc128);
+}
+
 int get_table(tgp_ctx* ctx, tgp_table_id id, const Table** out) {
     auto it = ctx->tables.find(id);
     if (it == ctx->tables.end()) return fail(ctx, TGP_NOT_FOUND, "unknown table id");
@@ -1784,7 +1941,8 @@ struct BucketSpec {
 // count, then per value two limbs of a sum, one word of a sum whose partial
 // in a CTA's table provably fits 32 bits, or one word of an extreme whose
 // value range is below 2^32. Returns the words per group, 0 when a value
-// has no such form. Fixed-shape value programs keep two words per value.
+// has no such form. Fixed-shape value programs keep two words per value: the
+// scan engine adds both limbs, of which a narrow sum's first alone counts.
 static uint32_t plan_s32_words(Builder& b, uint64_t rows, uint32_t sms, bool fixed_values) {
     Plan& P = b.P;
     // A CTA's tiles at any grid launch() takes (at least one CTA per SM, or
@@ -1804,9 +1962,9 @@ static uint32_t plan_s32_words(Builder& b, uint64_t rows, uint32_t sms, bool fix
             continue;
         }
         const unsigned __int128 most = static_cast<unsigned __int128>(std::max(abs128(b.val_lo[v]), abs128(b.val_hi[v])));
-        const bool narrow = !b.val_big[v] && !fixed_values && rows_cta * most < (static_cast<unsigned __int128>(1) << 31);
+        const bool narrow = !b.val_big[v] && rows_cta * most < (static_cast<unsigned __int128>(1) << 31);
         P.s32_kind[v] = narrow ? S32_NARROW : S32_WIDE;
-        w += narrow ? 1 : 2;
+        w += narrow && !fixed_values ? 1 : 2;
     }
     return w;
 }
@@ -1886,6 +2044,7 @@ static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t s
         uint64_t range = static_cast<uint64_t>(c.max) - static_cast<uint64_t>(c.min);
         if (bucket && k < bucket->nkeys) {
             K.lut = bucket->lut[k];
+            b.P.lut_cells[k] = static_cast<uint32_t>(std::min<uint64_t>(range + 1, 0xffffffffull));
             range = bucket->nbuckets[k] - 1;
         }
         dom[k] = range == ~0ull ? 0 : range + 1;  // 0 = full 64-bit domain
@@ -2470,10 +2629,7 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         direct_group_supported(P.slot[P.gkey[0].slot].dtype, P.nval ? P.slot[P.val[0].f[0].slot].dtype : 0u)) {
         TGP_TRY(launch_direct_groups(ctx, P, b.max_abs_val));
     } else {
-        bool done = false;
-        TGP_TRY(try_launch_q1(ctx, P, mode, acc128, ngroups_direct, b.max_abs_val, &done));
-        if (!done) TGP_TRY(try_launch_join(ctx, P, mode, ngroups_direct, &done));
-        if (!done) TGP_TRY(launch(ctx, P, mode, acc128));
+        TGP_TRY(launch_query(ctx, P, mode, acc128, ngroups_direct, b.max_abs_val));
     }
 
     const uint32_t nagg = q->nagg;
@@ -2594,6 +2750,8 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
     } else {
         TGP_TRY(pinned_reserve(ctx, back_words * 8 + 256 + (one_pass ? one_bytes : 0)));
         TGP_CUDA(cudaMemcpyAsync(ctx->hpin, block, back_words * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        if (one_pass && one_bytes)
+            TGP_CUDA(cudaMemcpyAsync(ctx->hpin + 256, fmt, one_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         TGP_CUDA(cudaStreamSynchronize(ctx->stream));
         hb = reinterpret_cast<const unsigned long long*>(ctx->hpin);
     }
@@ -2611,6 +2769,11 @@ static int execute_impl(tgp_ctx* ctx, const tgp_query* q, uint64_t* keys_out, tg
         const uint64_t ng = counters[2];
         result->ngroups = ng;
         if (ng > group_cap) return fail(ctx, TGP_CAPACITY, "group buffer too small");
+        if (one_pass) {
+            if (keys_out) std::memcpy(keys_out, ctx->hpin + 256, ng * q->ngroup * 8);
+            if (vals_out) std::memcpy(vals_out, ctx->hpin + 256 + one_keys, ng * nagg * sizeof(tgp_agg_value));
+            return TGP_OK;
+        }
         const HashFormat F = group_format();
         const size_t kbytes = (keys_out ? ng * q->ngroup * 8 : 0), vbytes = (vals_out ? ng * nagg * sizeof(tgp_agg_value) : 0);
         const size_t vofs = (kbytes + 255) & ~size_t{255};
@@ -2750,8 +2913,6 @@ int tgp_query_footprint(tgp_ctx* ctx, const tgp_query* q, uint64_t* device_bytes
     if (!ctx || !q || !device_bytes) return fail(ctx, TGP_INVALID_ARG, "null argument");
     QueryState qs;
     TGP_TRY(plan_query(ctx, q, qs, scan_kernel_static_smem(), nullptr, /*dry=*/true));
-        if (one_pass && one_bytes)
-            TGP_CUDA(cudaMemcpyAsync(ctx->hpin + 256, fmt, one_bytes, cudaMemcpyDeviceToHost, ctx->stream));
     plan_one_word_slots(qs, q, nullptr);
     const Plan& P = qs.b->P;
     // What execute_impl carves or allocates for one run of the query.
@@ -2769,11 +2930,6 @@ int tgp_query_footprint(tgp_ctx* ctx, const tgp_query* q, uint64_t* device_bytes
         }
         bytes += max_groups * (8ull * q->ngroup + sizeof(tgp_agg_value) * q->nagg) + 512;  // formatted result
     } else if (formats_direct(qs, q)) {
-        if (one_pass) {
-            if (keys_out) std::memcpy(keys_out, ctx->hpin + 256, ng * q->ngroup * 8);
-            if (vals_out) std::memcpy(vals_out, ctx->hpin + 256 + one_keys, ng * nagg * sizeof(tgp_agg_value));
-            return TGP_OK;
-        }
         bytes += direct_groups_scratch(qs.ngroups_direct) +
                  qs.ngroups_direct * (8ull * q->ngroup + sizeof(tgp_agg_value) * q->nagg) + 512;
     }
@@ -3878,14 +4034,13 @@ int tgp_batch_submit(tgp_ctx* ctx, tgp_batch_item* items, uint32_t n, tgp_batch_
     TGP_CUDA(cudaMemcpyAsync(B->dev, h, total, cudaMemcpyHostToDevice, ctx->stream));
     for (uint32_t i : solo) {
         const QueryState& qs = B->qs[i];
-        bool done = false;
-        TGP_TRY(try_launch_q1(ctx, qs.b->P, qs.mode, qs.acc128, qs.ngroups_direct, qs.b->max_abs_val, &done));
-        if (!done) TGP_TRY(try_launch_join(ctx, qs.b->P, qs.mode, qs.ngroups_direct, &done));
-        if (!done) TGP_TRY(launch(ctx, qs.b->P, qs.mode, qs.acc128));
+        TGP_TRY(launch_query(ctx, qs.b->P, qs.mode, qs.acc128, qs.ngroups_direct, qs.b->max_abs_val));
     }
     for (auto& M : B->merges) {
-        TGP_TRY(launch(ctx, M->qs.b->P, M->qs.mode, M->qs.acc128));
-        if (M->has_count) TGP_TRY(launch(ctx, M->cqs.b->P, M->cqs.mode, M->cqs.acc128));
+        TGP_TRY(launch_query(ctx, M->qs.b->P, M->qs.mode, M->qs.acc128, M->qs.ngroups_direct, M->qs.b->max_abs_val));
+        if (M->has_count)
+            TGP_TRY(launch_query(ctx, M->cqs.b->P, M->cqs.mode, M->cqs.acc128, M->cqs.ngroups_direct,
+                                 M->cqs.b->max_abs_val));
     }
     for (size_t k = 0; k < classes.size(); ++k) {
         const Class& c = classes[k];

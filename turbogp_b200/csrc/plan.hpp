@@ -301,6 +301,7 @@ struct alignas(16) Plan {
     uint32_t hpack_shift;
     int64_t hpack_bias;
     uint32_t jpay_w;
+    uint32_t lut_cells[kMaxGroupKeys];   // bucket keys: cells of GKey::lut
     const uint32_t* jbits;  // one bit per payload entry (a build row matches), or null
     ResultOut out;
     uint32_t two_ctas;      // launch the register budget of two CTAs per SM (join-payload limb-table shapes)

@@ -115,6 +115,49 @@ inline size_t join_stream_smem(uint32_t table_bytes, uint32_t copies, uint32_t n
 uint64_t pay_bits_words(uint64_t entries);
 cudaError_t launch_pay_bits(const uint8_t* pay, uint64_t entries, uint32_t* bits, int sms, cudaStream_t st);
 cudaError_t launch_join_stream(const JoinStreamArgs& A, bool bits, int grid, cudaStream_t st);
+// Streaming limb tables (group_stream.cu): a MODE_GROUP_SHARED32 plan whose
+// rows need no staging.
+constexpr int kGsKeys = 3, kGsCols = 3;
+enum { GS_COLS = 0, GS_Q1 = 1, GS_JOIN = 2 };                      // value programs
+enum { GS_PAY_NONE = 0, GS_PAY_BYTES = 1, GS_PAY_BITS = 2 };       // join payload lookups
+struct GroupStreamOp {
+    uint32_t off;             // byte offset of the value's words in a group's entry
+    uint32_t kind;            // S32_*
+    uint32_t slot;            // value slot of the query's accumulators (1 ..)
+    uint32_t nz;              // COUNT(col)
+    uint32_t ident;           // mul == 1 && add == 0
+    uint32_t ref;             // low word of ref64
+    int64_t ref64;            // Plan::s32_ref
+    int64_t mul, add;
+};
+struct GroupStreamArgs {
+    uint64_t nrows;
+    uint32_t nleaf, leaf_neg;
+    const uint8_t* leaf_col[4];
+    uint32_t leaf_lo[4], leaf_sp[4];
+    uint32_t nkey, ngroups;
+    struct {
+        const uint8_t* col;
+        const uint8_t* lut;   // bucket key: cells bytes, copied to lut_off
+        uint32_t dtype, min, stride, cells, lut_off, _pad;
+    } key[kGsKeys];
+    uint32_t ncol, nval;
+    struct {
+        const uint8_t* col;
+        uint32_t dtype, first, nops, _pad;   // ops first .. first + nops - 1 read this column (GS_COLS)
+    } col[4];                                // the fixed programs: price, then their int32 columns in order
+    GroupStreamOp op[kMaxVals];
+    uint32_t mul[3], add[3];                 // the fixed programs' int32 factors
+    const uint8_t* fk;                       // join: int32 probe key
+    const uint8_t* pay;
+    const void* table;
+    uint32_t table_bytes, kmin, krange;
+    uint32_t tab_off, words, copies, acc_stride, _pad;
+    unsigned long long* acc;
+    unsigned long long* counters;
+    ResultOut out;
+};
+cudaError_t launch_group_stream(const GroupStreamArgs& A, int vs, int pay, uint32_t smem, int grid, cudaStream_t st);
 bool hash_group_supported(uint32_t kdt, uint32_t vdt);
 uint64_t hash_group_grid(uint64_t nrows, int sms);
 uint64_t hash_group_rows_per_cta(uint64_t nrows, int sms);
@@ -215,6 +258,11 @@ cudaError_t count_direct_groups(const unsigned long long* htab, uint64_t nslots,
                                 size_t scratch_bytes, unsigned long long* total, cudaStream_t st);
 cudaError_t format_direct_groups(const unsigned long long* htab, uint64_t nslots, const void* scratch, uint64_t cap,
                                  const HashFormat& F, uint64_t* keys_out, tgp_agg_value* vals_out, cudaStream_t st);
+// The same in one pass over a table of at most kDirOneSlots slots; the outputs
+// have room for every slot.
+constexpr uint64_t kDirOneSlots = 32768;
+cudaError_t format_direct_one(const unsigned long long* htab, uint64_t nslots, const HashFormat& F, uint64_t* keys_out,
+                              tgp_agg_value* vals_out, unsigned long long* total, cudaStream_t st);
 // The first min(limit, n) gathered groups in the order of one aggregate
 // (ties in ascending key order), formatted like format_hash_groups.
 // Scratch: format_hash_groups_scratch(n, 64) bytes.
@@ -258,11 +306,6 @@ cudaError_t top_select_narrow(const unsigned long long* htab, uint64_t max_group
 cudaError_t launch_delay(uint64_t ns, cudaStream_t st);
 // Device-to-host copy by a kernel into page-locked (mapped) host memory; both
 // addresses and the size 16-byte aligned.
-// The same in one pass over a table of at most kDirOneSlots slots; the outputs
-// have room for every slot.
-constexpr uint64_t kDirOneSlots = 32768;
-cudaError_t format_direct_one(const unsigned long long* htab, uint64_t nslots, const HashFormat& F, uint64_t* keys_out,
-                              tgp_agg_value* vals_out, unsigned long long* total, cudaStream_t st);
 cudaError_t launch_copy_to_host(void* host_dst, const void* dev_src, size_t bytes, cudaStream_t st);
 cudaError_t launch_like(const uint8_t* bytes, const unsigned long long* offs, uint64_t n, const LikePattern& P,
                         bool negated, uint32_t* bitmap, unsigned long long* count, uint32_t* err, int sms,
