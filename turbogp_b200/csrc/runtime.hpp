@@ -404,6 +404,11 @@ struct tgp_ctx {
     // context's stream, so no cross-stream reuse dependency can chain two
     // contexts' work); null: the device's default pool.
     cudaMemPool_t pool = nullptr;
+    // Lanes beside `stream` for the independent launches of one batch: forked
+    // from it after the batch's upload, joined before its readback.
+    static constexpr int kLanes = 3;
+    cudaStream_t lane[kLanes] = {};
+    cudaEvent_t fork = nullptr, join[kLanes] = {};
     std::string err;
     std::unordered_map<uint64_t, tgp::Table> tables;
     std::unordered_map<uint64_t, tgp::JoinTable> joins;
