@@ -153,6 +153,33 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src_gmem, uint32_t 
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src_gmem), "r"(bytes) : "memory");
 }
 
+// Asks L2 for the line that holds `p` (global memory).
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
+}
+
+// L2 prefetch of a streaming kernel's later chunks: the columns' lines of one
+// warp chunk are dealt to the lanes (at most 32; later columns go without), and
+// each lane asks for its line of the chunk that the warp reads next. The
+// kernels' shared tables leave 16-32 warps per SM and few registers, too little
+// to cover HBM latency with loads; a chunk that is in L2 when it is read does
+// not need to be.
+struct LineAhead {
+    const uint8_t* at = nullptr;
+    uint32_t step = 0, used = 0;
+    __device__ __forceinline__ void column(uint32_t lane, const uint8_t* col, uint32_t chunk_bytes) {
+        const uint32_t n = chunk_bytes / 128u;
+        if (lane >= used && lane < used + n) {
+            at = col + (lane - used) * 128u;
+            step = chunk_bytes;
+        }
+        used += n;
+    }
+    __device__ __forceinline__ void fetch(uint64_t chunk) const {
+        if (at) prefetch_l2(at + chunk * step);
+    }
+};
+
 // L2 policy for data read exactly once: evict first.
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
     uint64_t p;

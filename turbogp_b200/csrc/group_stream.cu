@@ -10,6 +10,11 @@
 // tables, the bucket keys' per-cell tables (read through L1 they cost a tag
 // cycle per lane) and the join's payload bytes or match bits (join_stream.cu).
 // Rows in bucket 0 of a bucket key belong to no request and are left out.
+// B200, merged batch of 16 requests over 60M rows, scan engine -> here: scans
+// 314 -> 226 us, Q1 477 -> 328, joins 416 -> 282, the joins' count scan 173 -> 109;
+// 20M rows over 2,526 groups with extremes 211 -> 175. What bounds it is the
+// shared atomics: about three lanes of a warp on one bank, six to nine atomics
+// per row.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -194,8 +199,18 @@ __global__ void __launch_bounds__(kGsThreads, 1) group_stream_kernel(const __gri
     const uint64_t warp = static_cast<uint64_t>(blockIdx.x) * kGsWarps + wib;
     const uint64_t nwarps = static_cast<uint64_t>(gridDim.x) * kGsWarps;
     const uint64_t nfull = A.nrows / kGsRows;
+    // The next chunk's lines (the fixed programs; in the general one the shared
+    // atomics are the bound and the prefetch costs registers).
+    LineAhead ahead;
+    if (VS != GS_COLS) {
+        if (PAY != GS_PAY_NONE) ahead.column(lane, A.fk, 512);
+        for (uint32_t k = 0; k < A.nkey; ++k) ahead.column(lane, A.key[k].col, A.key[k].dtype == DT_U8 ? 128u : 512u);
+        for (uint32_t q = 0; q < (VS == GS_Q1 ? 4u : 2u); ++q) ahead.column(lane, A.col[q].col, q == 0 ? 1024u : 512u);
+        for (uint32_t i = 0; i < A.nleaf; ++i) ahead.column(lane, A.leaf_col[i], 512);
+    }
     for (uint64_t c = warp; c < nfull; c += nwarps) {
         const uint64_t r = c * kGsRows + 4 * lane;
+        if (VS != GS_COLS && c + nwarps < nfull) ahead.fetch(c + nwarps);
         // Every column's loads first.
         uint4 fk = make_uint4(0u, 0u, 0u, 0u), kx[kGsKeys];
         GsCells v[kGsCols];

@@ -129,6 +129,11 @@ __global__ void __launch_bounds__(kJsThreads, 1) join_stream_kernel(const JoinSt
         for (int e = 0; e < 4; ++e)
             if (k.g[e] != 0xffu) add(k.g[e], pp[e], dd[e]);
     };
+    LineAhead lines;
+    lines.column(lane, A.key, 512);
+    lines.column(lane, A.col0, 1024);
+    lines.column(lane, A.col1, 512);
+    for (uint32_t i = 0; i < A.nleaf; ++i) lines.column(lane, A.leaf_col[i], 512);
     if (warp < nfull) {
         Chunk a, b;
         uint4 key = load_key(warp), ahead = load_key(warp + nwarps);
@@ -136,6 +141,8 @@ __global__ void __launch_bounds__(kJsThreads, 1) join_stream_kernel(const JoinSt
         for (uint64_t c = warp;; c += 2 * nwarps) {
             const uint64_t c1 = c + nwarps, c2 = c1 + nwarps;
             key = ahead;
+            if (c2 < nfull) lines.fetch(c2);
+            if (c2 + nwarps < nfull) lines.fetch(c2 + nwarps);
             ahead = load_key(c2);
             if (c1 < nfull) start(c1, key, b);
             finish(a);
