@@ -1971,7 +1971,9 @@ static uint32_t plan_s32_words(Builder& b, uint64_t rows, uint32_t sms, bool fix
         P.s32_kind[v] = narrow ? S32_NARROW : S32_WIDE;
         w += narrow && !fixed_values ? 1 : 2;
     }
-    return w;
+    // An odd number of words, so that one value's words of random groups fall
+    // on all 32 banks (an even one halves them).
+    return w | 1u;
 }
 
 static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t static_smem,

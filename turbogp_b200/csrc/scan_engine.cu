@@ -871,31 +871,30 @@ struct Sink {
                 // Sum the copies' limbs: counts as u64; a wide value as the
                 // exact int64 (hi << 32) + lo of each copy; extremes as the
                 // maximum over the copies, of a group with rows.
+                const size_t step = static_cast<size_t>(G) * W;
+                const uint32_t* e = tab + static_cast<size_t>(g) * W + (v == 0 ? 0u : P.s32_off[v - 1]);
                 int64_t sum = 0;
-                uint32_t far = 0, rows = 0;
-                for (uint32_t c = 0; c < P.s32_copies; ++c) {
-                    const uint32_t* e = tab + (static_cast<size_t>(c) * G + g) * W;
-                    if (v == 0) {
-                        sum += static_cast<int64_t>(e[0]);
-                        continue;
-                    }
-                    rows |= e[0];
-                    e += P.s32_off[v - 1];
-                    if (sk == S32_WIDE) {
-                        const uint64_t hi = static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(e[1])));
-                        sum = static_cast<int64_t>(static_cast<uint64_t>(sum) + ((hi << 32) | e[0]));
-                    } else if (sk == S32_NARROW) {
-                        sum += static_cast<int64_t>(static_cast<int32_t>(e[0]));
-                    } else {
-                        far = max(far, e[0]);
-                    }
-                }
                 if (sk == S32_MIN || sk == S32_MAX) {
+                    uint32_t far = 0, rows = 0;
+                    for (uint32_t c = 0; c < P.s32_copies; ++c) {
+                        far = max(far, e[c * step]);
+                        rows |= tab[c * step + static_cast<size_t>(g) * W];
+                    }
                     if (rows == 0) continue;
                     const int64_t x = sk == S32_MIN ? P.s32_ref[v - 1] - static_cast<int64_t>(far)
                                                     : P.s32_ref[v - 1] + static_cast<int64_t>(far);
                     acc_global_i64(P.acc + 2ull * idx, sk == S32_MIN ? VK_MIN : VK_MAX, x);
                     continue;
+                }
+                for (uint32_t c = 0; c < P.s32_copies; ++c, e += step) {
+                    if (v == 0) {
+                        sum += static_cast<int64_t>(e[0]);
+                    } else if (sk == S32_WIDE) {
+                        const uint64_t hi = static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(e[1])));
+                        sum = static_cast<int64_t>(static_cast<uint64_t>(sum) + ((hi << 32) | e[0]));
+                    } else {
+                        sum += static_cast<int64_t>(static_cast<int32_t>(e[0]));
+                    }
                 }
                 if (sum == 0) continue;
                 I128 a;
