@@ -5,8 +5,8 @@ import numpy as np
 import pytest
 
 import oracle
-from turbogp_b200 import datagen
-from turbogp_b200.engine import avg, col, count_col, count_star, max_, min_, sum_
+from turbogp_b200 import datagen, workloads
+from turbogp_b200.engine import Context, avg, col, count_col, count_star, max_, min_, sum_
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +91,16 @@ def test_limb_tables_of_sums_and_extremes(ctx, n, groups):
     same(ctx.submit([pq, t.prepare(shapes[4], ("key",), None, group_cap=16_384)]).wait()[1],
          oracle.aggregate(h, None, shapes[4], ("key",), None))
     t.drop()
+
+
+def test_autotuner_times_launches_whose_results_are_handed_over():
+    """A result handed over by the kernel is read before the launch has
+    ended: the tuner waits for the launch before it reads its time."""
+    host = datagen.lineitem(400_000, seed=77)
+    with Context(0) as ctx:
+        t = ctx.register(host, datagen.LINEITEM_COLTYPES)
+        for tpl in (workloads.filtered_group_agg(), workloads.selective_scan_sum()):
+            rep = ctx.autotune(t.prepare(tpl.aggs, tpl.group_by, tpl.where), reps=3)
+            ran = [c for c in rep["candidates"] if c["status"] == 0 and c["same_result"]]
+            assert ran and all(c["ms"] > 0 for c in ran)
+        t.drop()

@@ -760,7 +760,8 @@ int size_smem(tgp_ctx* ctx, Plan& P, size_t extra_bytes, size_t static_smem = sc
     // value program run two CTAs of 512 threads and two stages per SM (34
     // warps instead of 17 to hide the payload lookups; 60M x 1.5M probe
     // 0.164 -> 0.140 ms at 30M probe rows), unless a variant caps the stages
-    // and keeps one CTA.
+    // and keeps one CTA. Key ranges whose bytes or bits fit a CTA's shared
+    // memory run join_stream_kernel or group_stream_kernel instead.
     P.two_ctas = (P.jpay != nullptr && P.s32_copies != 0 && P.shape != 0 && P.nthreads == 512 && stage &&
                   (K.ctas_per_sm == 2 || K.max_stages >= kMaxStages)) ? 1u : 0u;
     if (P.two_ctas) {
@@ -3254,8 +3255,10 @@ int tgp_autotune(tgp_ctx* ctx, const tgp_query* q, uint32_t reps, tgp_tune_entry
                 e.status = run_into(ctx, q, &r);
                 double ms = 0.0;
                 for (size_t j = 0; j < ctx->prof_used; ++j) {
+                    // A handed-over result is read before the launch has ended.
                     float f = 0.f;
-                    if (cudaEventElapsedTime(&f, ctx->prof_events[j].first, ctx->prof_events[j].second) == cudaSuccess)
+                    if (cudaEventSynchronize(ctx->prof_events[j].second) == cudaSuccess &&
+                        cudaEventElapsedTime(&f, ctx->prof_events[j].first, ctx->prof_events[j].second) == cudaSuccess)
                         ms += f;
                 }
                 t.push_back(ms);
