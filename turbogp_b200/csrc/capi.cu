@@ -36,6 +36,29 @@ inline bool pay_bytes_fit(uint64_t entries) { return entries <= kPayBytesMax; }
 inline bool pay_bits_fit(uint64_t entries, uint32_t width) {
     return width == 1 && !pay_bytes_fit(entries) && entries <= kPayBitsMax;
 }
+
+// The lookup of a streaming join: int32 probe keys through a payload of one
+// byte per key, whose bytes or match bits a CTA keeps in shared memory. The
+// kernels take a probe key's distance from the smallest build key in 32 bits,
+// which is the 64-bit distance only when every build key is an int32 value too
+// (build keys may be int64: past int32 a probe key would meet the build key
+// 2^32 away). table = null: not such a join, the scan engine compares in 64 bits.
+struct StreamLookup {
+    const void* table = nullptr;
+    uint32_t table_bytes = 0;   // whole 16-byte words
+    bool bits = false;
+};
+StreamLookup stream_lookup(const Plan& P) {
+    StreamLookup L;
+    if (P.jslot < 0 || !P.jpay || P.jpay_w != 1 || P.slot[P.jslot].dtype != DT_I32 || P.jkmin < INT32_MIN ||
+        P.jkmin > INT32_MAX || P.jkrange > static_cast<uint64_t>(INT32_MAX - P.jkmin))
+        return L;
+    const uint64_t entries = P.jkrange + 1;
+    L.bits = !pay_bytes_fit(entries);
+    L.table = L.bits ? static_cast<const void*>(P.jbits) : static_cast<const void*>(P.jpay);
+    L.table_bytes = static_cast<uint32_t>(L.bits ? pay_bits_words(entries) * 4 : (entries + 15) & ~uint64_t{15});
+    return L;
+}
 constexpr size_t kJoinSmemCap = 144u << 10;        // shared memory per CTA of a payload-join scan (see size_smem)
 
 int fail(tgp_ctx* ctx, int st, const std::string& m) {
@@ -1034,21 +1057,19 @@ int try_launch_q1(tgp_ctx* ctx, const Plan& P, uint32_t mode, bool acc128, uint6
 // us); fewer rows stay with the scan engine.
 int try_launch_join(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroups, bool* done) {
     *done = false;
-    if (ctx->dbg_skip_tile1 || mode != MODE_GROUP_SHARED32 || P.shape != kShapeJoin || !P.dense_vec || !P.jpay ||
-        P.jpay_w != 1 || !P.sum64 || P.check_ovf || P.nval != 1 || P.chain.nsteps != 2 || ngroups == 0 || ngroups > 254 ||
-        P.jslot < 0 || P.slot[P.jslot].dtype != DT_I32 || P.jkrange >= 0xffffffffull)
+    if (ctx->dbg_skip_tile1 || mode != MODE_GROUP_SHARED32 || P.shape != kShapeJoin || !P.dense_vec || !P.sum64 ||
+        P.check_ovf || P.nval != 1 || P.chain.nsteps != 2 || ngroups == 0 || ngroups > 254)
         return TGP_OK;
+    const StreamLookup look = stream_lookup(P);
+    if (!look.table) return TGP_OK;
     if (P.nleaf > 4 || (P.nleaf && !(P.all_and && P.kend[0] == P.nleaf))) return TGP_OK;
     for (uint32_t k = 0; k < P.ngkey; ++k)
         if (!P.gkey[k].build_side || P.gkey[k].lut) return TGP_OK;
-    const uint64_t entries = P.jkrange + 1;
-    const bool bytes = pay_bytes_fit(entries);
-    const size_t budget = bytes ? ctx->max_dyn_smem - 1024 : kPayBitsSmem;
-    if (!bytes && !P.jbits) return TGP_OK;
+    const size_t budget = look.bits ? kPayBitsSmem : ctx->max_dyn_smem - 1024;
     JoinStreamArgs A;
     std::memset(&A, 0, sizeof(A));
-    A.table = bytes ? static_cast<const void*>(P.jpay) : static_cast<const void*>(P.jbits);
-    A.table_bytes = static_cast<uint32_t>(bytes ? (entries + 15) & ~uint64_t{15} : pay_bits_words(entries) * 4);
+    A.table = look.table;
+    A.table_bytes = look.table_bytes;
     A.ngroups = static_cast<uint32_t>(ngroups);
     A.copies = 32;   // one per warp
     while (A.copies > 1 && join_stream_smem(A.table_bytes, A.copies, A.ngroups) > budget) A.copies >>= 1;
@@ -1083,7 +1104,7 @@ int try_launch_join(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroups
     A.out = P.out;
     std::pair<cudaEvent_t, cudaEvent_t>* ev = nullptr;
     TGP_TRY(profile_begin(ctx, &ev));
-    const cudaError_t e = launch_join_stream(A, !bytes, static_cast<int>(grid), ctx->stream);
+    const cudaError_t e = launch_join_stream(A, look.bits, static_cast<int>(grid), ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("join launch: ") + cudaGetErrorString(e));
     if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
     *done = true;
@@ -1112,13 +1133,11 @@ int try_launch_group(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroup
     uint32_t off = 0;   // shared memory taken so far
     int pay = GS_PAY_NONE;
     if (P.jslot >= 0) {
-        if (!P.jpay || P.jpay_w != 1 || P.slot[P.jslot].dtype != DT_I32 || P.jkrange >= 0xffffffffull) return TGP_OK;
-        const uint64_t entries = P.jkrange + 1;
-        const bool bytes = pay_bytes_fit(entries);
-        if (!bytes && !P.jbits) return TGP_OK;
-        pay = bytes ? GS_PAY_BYTES : GS_PAY_BITS;
-        A.table = bytes ? static_cast<const void*>(P.jpay) : static_cast<const void*>(P.jbits);
-        A.table_bytes = static_cast<uint32_t>(bytes ? (entries + 15) & ~uint64_t{15} : pay_bits_words(entries) * 4);
+        const StreamLookup look = stream_lookup(P);
+        if (!look.table) return TGP_OK;
+        pay = look.bits ? GS_PAY_BITS : GS_PAY_BYTES;
+        A.table = look.table;
+        A.table_bytes = look.table_bytes;
         A.fk = P.slot[P.jslot].ptr;
         A.pay = reinterpret_cast<const uint8_t*>(P.jpay);
         A.kmin = static_cast<uint32_t>(P.jkmin);
