@@ -1240,8 +1240,7 @@ int try_launch_group(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroup
     if (off + entry > budget) return TGP_OK;
     A.copies = 32;
     while (A.copies > 1 && off + A.copies * entry > budget) A.copies >>= 1;
-    const uint64_t chunks = (P.nrows + 127) / 128;
-    const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((chunks + 31) / 32, static_cast<uint64_t>(ctx->sms)));
+    const uint64_t grid = group_stream_grid(P.nrows, ctx->sms);
     // The tables are filled, cleared and merged once per CTA.
     if (P.nrows / grid < (off + entry) / 16) return TGP_OK;
     A.acc = P.acc;
@@ -1999,11 +1998,14 @@ struct BucketSpec {
 // scan engine adds both limbs, of which a narrow sum's first alone counts.
 static uint32_t plan_s32_words(Builder& b, uint64_t rows, uint32_t sms, bool fixed_values) {
     Plan& P = b.P;
-    // A CTA's tiles at any grid launch() takes (at least one CTA per SM, or
-    // one per tile): its tables' rows.
+    // The most rows of one CTA, all of which may fall into one word: of the
+    // scan engine at any grid launch() takes (at least one CTA per SM, or one
+    // per tile), or of the streaming kernel, whichever runs the plan. (Five
+    // tiles per SM are 10,240 rows there and 12,288 here.)
     const uint64_t ntiles = (rows + kTileRows - 1) / kTileRows;
     const uint64_t ctas = std::max<uint64_t>(1, std::min<uint64_t>(ntiles, sms));
-    const unsigned __int128 rows_cta = static_cast<unsigned __int128>((ntiles + ctas - 1) / ctas) * kTileRows;
+    const unsigned __int128 rows_cta = std::min<uint64_t>(
+        rows, std::max<uint64_t>((ntiles + ctas - 1) / ctas * kTileRows, group_stream_rows_per_cta(rows, static_cast<int>(sms))));
     uint32_t w = 1;
     for (uint32_t v = 0; v < P.nval; ++v) {
         const uint8_t kind = P.val[v].kind;

@@ -17,6 +17,7 @@
 // per row.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "device_common.cuh"
@@ -361,6 +362,17 @@ const void* gs_kernel(int pay) {
 }
 
 }  // namespace
+
+uint64_t group_stream_grid(uint64_t nrows, int sms) {
+    const uint64_t chunks = (nrows + kGsRows - 1) / kGsRows;
+    return std::max<uint64_t>(1, std::min<uint64_t>((chunks + kGsWarps - 1) / kGsWarps, static_cast<uint64_t>(sms)));
+}
+
+uint64_t group_stream_rows_per_cta(uint64_t nrows, int sms) {
+    // Warp c % warps takes chunk c, the partial last one included.
+    const uint64_t chunks = (nrows + kGsRows - 1) / kGsRows, nwarps = group_stream_grid(nrows, sms) * kGsWarps;
+    return (chunks + nwarps - 1) / nwarps * kGsRows * kGsWarps;
+}
 
 cudaError_t launch_group_stream(const GroupStreamArgs& A, int vs, int pay, uint32_t smem, int grid, cudaStream_t st) {
     const void* f = vs == GS_COLS ? gs_kernel<GS_COLS>(pay) : vs == GS_Q1 ? gs_kernel<GS_Q1>(pay) : gs_kernel<GS_JOIN>(pay);

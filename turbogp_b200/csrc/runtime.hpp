@@ -157,6 +157,10 @@ struct GroupStreamArgs {
     unsigned long long* counters;
     ResultOut out;
 };
+// The kernel's grid, and the most rows of one CTA at that grid (the bound of a
+// one-word sum: plan_s32_words).
+uint64_t group_stream_grid(uint64_t nrows, int sms);
+uint64_t group_stream_rows_per_cta(uint64_t nrows, int sms);
 cudaError_t launch_group_stream(const GroupStreamArgs& A, int vs, int pay, uint32_t smem, int grid, cudaStream_t st);
 bool hash_group_supported(uint32_t kdt, uint32_t vdt);
 uint64_t hash_group_grid(uint64_t nrows, int sms);
