@@ -252,26 +252,33 @@ __device__ __forceinline__ int64_t add_wrap_checked(int64_t a, int64_t b, uint32
 // by `nt` threads of every CTA (t = 0 .. nt - 1) after their last update of the
 // result block; `bar` is a barrier over those threads.
 // ---------------------------------------------------------------------------
+// Order: a barrier gathers the CTA's updates behind thread 0, whose fence then
+// covers them all (fences are cumulative) before its ticket; the last CTA's
+// thread 0 fences again between the ticket and the barrier that lets the others
+// read. In the same way thread 0 stores the sequence word behind a barrier and a
+// system fence of its own, so the host that sees it sees every word before it.
 template <typename BAR>
 __device__ __forceinline__ void finish_result(const ResultOut& O, uint32_t t, uint32_t nt, BAR&& bar) {
     if (!O.host) return;
     __shared__ uint32_t last;
-    __threadfence();   // this thread's updates are performed before its CTA counts as done
     bar();
-    if (t == 0) last = atomicAdd(O.ticket, 1u) == gridDim.x - 1u ? 1u : 0u;
+    if (t == 0) {
+        __threadfence();
+        last = atomicAdd(O.ticket, 1u) == gridDim.x - 1u ? 1u : 0u;
+        __threadfence();
+    }
     bar();
     if (!last) return;
-    __threadfence();
     ulonglong2* blk = reinterpret_cast<ulonglong2*>(O.block);
     ulonglong2* dst = reinterpret_cast<ulonglong2*>(O.host);
     for (uint32_t i = t; i < O.words16; i += nt) {
         dst[i] = __ldcg(blk + i);
         blk[i] = make_ulonglong2(0ull, 0ull);
     }
-    __threadfence_system();
     bar();
     if (t == 0) {
         *O.ticket = 0;
+        __threadfence_system();
         *reinterpret_cast<volatile unsigned long long*>(O.host + 2ull * O.words16) = O.seq;
     }
 }
