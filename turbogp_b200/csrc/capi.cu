@@ -16,6 +16,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "batch_lanes.hpp"
 #include "runtime.hpp"
 
 using namespace tgp;
@@ -3428,60 +3429,6 @@ void tgp_batch_free_rec(tgp_ctx* ctx, void* r) {
     delete B;
 }
 
-// The lanes of one batch's small launches (fewer tiles than SMs: 15-20 us each
-// of mostly latency, most SMs idle): next() gives the stream of the following
-// one in turn (the context's own among them), by pointing ctx->stream at it;
-// join() puts the context's stream back, behind every lane. Launches that fill
-// the SMs stay one after another: their CTAs split the rows evenly and expect
-// to start together, and side by side (three queries over 22M-30M rows) took
-// 0.39 ms instead of 0.34. Off while launches are profiled (their events
-// bracket one stream).
-class BatchLanes {
-  public:
-    explicit BatchLanes(tgp_ctx* c, size_t launches) : ctx(c), main(c->stream) {
-        if (launches < 3 || c->profile) return;
-        bool ok = c->fork || cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) == cudaSuccess;
-        for (int i = 0; ok && i < tgp_ctx::kLanes; ++i)
-            ok = (c->lane[i] || cudaStreamCreateWithFlags(&c->lane[i], cudaStreamNonBlocking) == cudaSuccess) &&
-                 (c->join[i] || cudaEventCreateWithFlags(&c->join[i], cudaEventDisableTiming) == cudaSuccess);
-        if (!ok || cudaEventRecord(c->fork, main) != cudaSuccess) {
-            cudaGetLastError();
-            return;
-        }
-        on = true;
-    }
-    ~BatchLanes() { join(); }
-    void next() {
-        if (!on) return;
-        at = (at + 1) % (tgp_ctx::kLanes + 1);
-        ctx->stream = at == 0 ? main : ctx->lane[at - 1];
-        if (at && !used[at - 1]) {
-            used[at - 1] = true;
-            cudaStreamWaitEvent(ctx->stream, ctx->fork, 0);
-        }
-    }
-    // False when a lane could not be joined (its work may still run).
-    bool join() {
-        ctx->stream = main;
-        bool ok = true;
-        for (int i = 0; i < tgp_ctx::kLanes; ++i) {
-            if (!used[i]) continue;
-            used[i] = false;
-            if (cudaEventRecord(ctx->join[i], ctx->lane[i]) != cudaSuccess ||
-                cudaStreamWaitEvent(main, ctx->join[i], 0) != cudaSuccess)
-                ok = cudaStreamSynchronize(ctx->lane[i]) == cudaSuccess && ok;
-        }
-        return ok;
-    }
-
-  private:
-    tgp_ctx* ctx;
-    cudaStream_t main;
-    bool on = false;
-    bool used[tgp_ctx::kLanes] = {};
-    int at = -1;
-};
-
 static size_t align256(size_t x) { return (x + 255) & ~size_t{255}; }
 
 // Whether a cell passes a comparison leaf with its column's comparison type
@@ -4151,7 +4098,7 @@ int tgp_batch_submit(tgp_ctx* ctx, tgp_batch_item* items, uint32_t n, tgp_batch_
     for (uint32_t i : solo)
         (B->qs[i].b->P.nrows <= static_cast<uint64_t>(ctx->sms) * kTileRows ? small : large).push_back(i);
     {
-        BatchLanes lanes(ctx, small.size());
+        BatchLanes<tgp_ctx> lanes(ctx, small.size());
         for (uint32_t i : small) {
             const QueryState& qs = B->qs[i];
             lanes.next();
