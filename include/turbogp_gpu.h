@@ -85,6 +85,13 @@ TGP_API int tgp_ctx_sm_count(const tgp_ctx* ctx);
 /* Blocks until all work enqueued on the context's stream has finished. */
 TGP_API int tgp_sync(tgp_ctx* ctx);
 
+/* Page-locks host memory of the caller's for every CUDA context of the process,
+ * so that results are copied into it at link speed, and unlocks it again
+ * (before the memory is freed). The calling thread's current device is used:
+ * the one tgp_init selected. */
+TGP_API int tgp_host_lock(void* p, uint64_t bytes);
+TGP_API int tgp_host_unlock(void* p);
+
 /* When enabled, the context records CUDA events on its stream around every
  * scan-kernel launch; tgp_profile_read returns the launches recorded since the
  * last read and their summed device time (ms), then resets the record.

@@ -279,6 +279,8 @@ extern "C" {
     pub fn tgp_ctx_stream(ctx: *mut tgp_ctx) -> *mut c_void;
     pub fn tgp_ctx_sm_count(ctx: *const tgp_ctx) -> c_int;
     pub fn tgp_sync(ctx: *mut tgp_ctx) -> c_int;
+    pub fn tgp_host_lock(p: *mut c_void, bytes: u64) -> c_int;
+    pub fn tgp_host_unlock(p: *mut c_void) -> c_int;
     pub fn tgp_profile_enable(ctx: *mut tgp_ctx, on: c_int) -> c_int;
     pub fn tgp_profile_read(ctx: *mut tgp_ctx, launches: *mut u64, total_ms: *mut f64) -> c_int;
 

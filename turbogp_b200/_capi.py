@@ -136,6 +136,8 @@ PROTOTYPES = [
     ("tgp_ctx_stream", C.c_void_p, [C.c_void_p]),
     ("tgp_ctx_sm_count", C.c_int, [C.c_void_p]),
     ("tgp_sync", C.c_int, [C.c_void_p]),
+    ("tgp_host_lock", C.c_int, [C.c_void_p, C.c_uint64]),
+    ("tgp_host_unlock", C.c_int, [C.c_void_p]),
     ("tgp_profile_enable", C.c_int, [C.c_void_p, C.c_int]),
     ("tgp_profile_read", C.c_int, [C.c_void_p, C.POINTER(C.c_uint64), C.POINTER(C.c_double)]),
     ("tgp_kernel_count", C.c_uint32, []),

@@ -1440,6 +1440,20 @@ int tgp_shutdown(tgp_ctx* ctx) {
     return TGP_OK;
 }
 
+int tgp_host_lock(void* p, uint64_t bytes) {
+    if (!p || !bytes) return TGP_INVALID_ARG;
+    if (cudaHostRegister(p, bytes, cudaHostRegisterPortable) == cudaSuccess) return TGP_OK;
+    cudaGetLastError();
+    return TGP_OOM;
+}
+
+int tgp_host_unlock(void* p) {
+    if (!p) return TGP_INVALID_ARG;
+    if (cudaHostUnregister(p) == cudaSuccess) return TGP_OK;
+    cudaGetLastError();
+    return TGP_INVALID_ARG;
+}
+
 const char* tgp_last_error(const tgp_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 
 void* tgp_ctx_stream(tgp_ctx* ctx) { return ctx ? static_cast<void*>(ctx->stream) : nullptr; }

@@ -296,27 +296,25 @@ class _PinnedPool:
             if self._bytes + size > self.LIMIT:
                 return None
             self._bytes += size
-        buf = self._register(size)
-        if buf is None:
-            with self._lock:
-                self._bytes -= size
-            return None
-        return np.asarray(_PinnedLease(self, buf))
+        buf = None
+        try:
+            buf = self._register(size)
+        except Exception:   # no memory, no library: an ordinary array serves
+            pass
+        finally:
+            if buf is None:
+                with self._lock:
+                    self._bytes -= size
+        return None if buf is None else np.asarray(_PinnedLease(self, buf))
 
     @staticmethod
     def _register(size: int) -> np.ndarray | None:
-        import torch
-        if not torch.cuda.is_available():
-            return None
         buf = np.empty(size, dtype=np.uint8)
-        if int(torch.cuda.cudart().cudaHostRegister(buf.ctypes.data, size, 1)) != 0:
-            return None
-        return buf
+        return buf if A.load().tgp_host_lock(buf.ctypes.data, size) == A.OK else None
 
     @staticmethod
     def _unregister(buf: np.ndarray) -> None:
-        import torch
-        torch.cuda.cudart().cudaHostUnregister(buf.ctypes.data)
+        A.load().tgp_host_unlock(buf.ctypes.data)
 
     def _give(self, buf: np.ndarray) -> None:
         with self._lock:
