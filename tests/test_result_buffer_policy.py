@@ -1,0 +1,81 @@
+"""When a large result gets a page-locked buffer, on the CPU with the locking
+counted: never for results that are kept or larger than the pool keeps idle,
+once for results that are dropped, whatever else lies idle."""
+import numpy as np
+import pytest
+
+from turbogp_b200 import engine
+
+MB = 1 << 20
+
+
+@pytest.fixture
+def pool(monkeypatch):
+    p = engine._PinnedPool()
+    p.locked, p.unlocked = [], []
+
+    def register(size):
+        p.locked.append(size)
+        return np.empty(size, dtype=np.uint8)
+    monkeypatch.setattr(p, "_register", register, raising=False)
+    monkeypatch.setattr(p, "_unregister", lambda buf: p.unlocked.append(buf.nbytes), raising=False)
+    monkeypatch.setattr(engine, "_PINNED", p)
+    return p
+
+
+def array(nbytes):
+    return engine._result_array(nbytes // 4, np.uint32)
+
+
+def test_kept_results_lock_nothing(pool):
+    kept = [array(12 * MB) for _ in range(20)]
+    assert pool.locked == [] and len({a.ctypes.data for a in kept}) == 20
+
+
+def test_dropped_results_lock_once(pool):
+    for _ in range(20):
+        array(12 * MB)
+    assert pool.locked == [12 * MB] and pool.unlocked == []
+    keep = [array(12 * MB) for _ in range(20)]   # the one buffer, then ordinary arrays
+    assert pool.locked == [12 * MB]
+    del keep
+    assert pool._bytes == pool._idle_bytes == 12 * MB
+
+
+def test_a_window_of_kept_results_ends_on_locked_buffers(pool):
+    window = []
+    for _ in range(40):
+        window.append(array(8 * MB))
+        del window[:-4]
+    assert pool.locked == [8 * MB] * 5 and pool.unlocked == []
+
+
+@pytest.mark.parametrize("nbytes", [256 * MB + 4, 400 * MB])
+def test_results_above_the_idle_bound_are_ordinary(pool, nbytes):
+    for _ in range(4):
+        array(nbytes)
+    assert pool.locked == [] and pool._bytes == 0 and not pool._dropped
+
+
+def test_small_idle_buffers_make_room(pool):
+    held = [pool.take(16 * MB) for _ in range(16)]
+    del held
+    assert pool._idle_bytes == pool.KEEP
+    for _ in range(6):
+        array(48 * MB)
+    assert pool.locked[16:] == [48 * MB]         # locked once although the bound was reached
+    assert pool.unlocked == [16 * MB] * 3 and pool._idle_bytes <= pool.KEEP
+
+
+def test_idle_buffers_make_room_below_the_limit(pool):
+    held = [pool.take(192 * MB) for _ in range(5)]
+    held.pop()
+    assert pool._bytes == 960 * MB and pool._idle_bytes == 192 * MB
+    assert pool.take(128 * MB) is not None       # 1,088 MB with the idle one
+    assert pool.unlocked == [192 * MB]
+
+
+@pytest.mark.parametrize("nbytes", [MB, MB + 1, 3 * MB, 5 * MB + 17, 130 * MB, 256 * MB - 1, 256 * MB])
+def test_buffers_waste_at_most_a_quarter(pool, nbytes):
+    size = pool._size(nbytes)
+    assert nbytes <= size <= nbytes * 1.25 and pool._size(size) == size

@@ -270,9 +270,15 @@ class _PinnedPool:
     """Page-locked buffers behind large result arrays. A device-to-host copy
     into fresh pageable memory runs at the speed at which the host can map and
     clear pages (a few GB/s on one thread); into a page-locked buffer it runs
-    at link speed. An array holds its buffer until it and every view of it are
-    gone; then the buffer serves the next result. All buffers together stay
-    within LIMIT bytes and the idle ones within KEEP (the rest is unlocked and
+    at link speed, but locking one costs as much as the copy it speeds up, so
+    it pays from its second result on. A program that drops its results gets
+    one buffer locked per result of that size it dropped; one that keeps them
+    gets ordinary arrays, and so does any result above KEEP, whose buffer
+    could not wait for the next one.
+
+    An array holds its buffer until it and every view of it are gone; then the
+    buffer serves the next result. All buffers together stay within LIMIT bytes
+    and the idle ones within KEEP (the ones idle longest are unlocked and
     freed); past LIMIT, or without a device, results are ordinary arrays."""
 
     MIN = 1 << 20
@@ -281,21 +287,42 @@ class _PinnedPool:
 
     def __init__(self):
         self._lock = threading.RLock()   # re-entered when a collection inside a call drops an array
-        self._idle: dict[int, list] = {}
+        self._idle: list[np.ndarray] = []   # longest idle first
         self._idle_bytes = self._bytes = 0
+        self._dropped: set[int] = set()   # buffer sizes of which an ordinary array was dropped
+
+    @staticmethod
+    def _size(nbytes: int) -> int:
+        """The buffer size for nbytes: a power of two, or one in quarter steps between."""
+        step = 1 << max((nbytes - 1).bit_length() - 3, 0)
+        return -(-nbytes // step) * step
+
+    def result(self, nbytes: int) -> np.ndarray:
+        """A uint8 array of at least nbytes for one result."""
+        size = self._size(nbytes)
+        with self._lock:
+            locked = size <= self.KEEP and (size in self._dropped or any(b.nbytes == size for b in self._idle))
+            if locked and not any(b.nbytes == size for b in self._idle):
+                self._dropped.discard(size)
+        raw = self.take(nbytes) if locked else None
+        return np.asarray(_OrdinaryLease(self, np.empty(nbytes, dtype=np.uint8), size)) if raw is None else raw
 
     def take(self, nbytes: int) -> np.ndarray | None:
-        """A uint8 array of at least nbytes, or None."""
-        size = 1 << (nbytes - 1).bit_length()
+        """A page-locked uint8 array of at least nbytes, or None."""
+        size = self._size(nbytes)
         with self._lock:
-            free = self._idle.get(size)
-            if free:
-                buf = free.pop()
-                self._idle_bytes -= size
-                return np.asarray(_PinnedLease(self, buf))
-            if self._bytes + size > self.LIMIT:
-                return None
-            self._bytes += size
+            for i in range(len(self._idle) - 1, -1, -1):
+                if self._idle[i].nbytes == size:
+                    buf = self._idle.pop(i)
+                    self._idle_bytes -= size
+                    return np.asarray(_PinnedLease(self, buf))
+            room = self._trim(self.KEEP, self.LIMIT - size)
+            fits = self._bytes + size <= self.LIMIT
+            if fits:
+                self._bytes += size
+        self._free(room)
+        if not fits:
+            return None
         buf = None
         try:
             buf = self._register(size)
@@ -316,14 +343,26 @@ class _PinnedPool:
     def _unregister(buf: np.ndarray) -> None:
         A.load().tgp_host_unlock(buf.ctypes.data)
 
+    def _trim(self, idle: int, total: int) -> list:
+        """Takes the longest idle buffers out until the bounds hold, or none is idle."""
+        out = []
+        while self._idle and (self._idle_bytes > idle or self._bytes > total):
+            buf = self._idle.pop(0)
+            self._idle_bytes -= buf.nbytes
+            self._bytes -= buf.nbytes
+            out.append(buf)
+        return out
+
+    def _free(self, bufs: list) -> None:
+        for buf in bufs:
+            self._unregister(buf)
+
     def _give(self, buf: np.ndarray) -> None:
         with self._lock:
-            if self._idle_bytes + buf.nbytes <= self.KEEP:
-                self._idle.setdefault(buf.nbytes, []).append(buf)
-                self._idle_bytes += buf.nbytes
-                return
-            self._bytes -= buf.nbytes
-        self._unregister(buf)
+            self._idle.append(buf)
+            self._idle_bytes += buf.nbytes
+            out = self._trim(self.KEEP, self.LIMIT)
+        self._free(out)
 
 
 class _PinnedLease:
@@ -339,6 +378,19 @@ class _PinnedLease:
             self._pool._give(self._buf)
 
 
+class _OrdinaryLease(_PinnedLease):
+    """The owner of an ordinary array: tells the pool that results of its size
+    are dropped."""
+
+    def __init__(self, pool: _PinnedPool, buf: np.ndarray, size: int):
+        super().__init__(pool, buf)
+        self._size = size
+
+    def __del__(self):
+        if sys is not None and not sys.is_finalizing() and self._size <= self._pool.KEEP:
+            self._pool._dropped.add(self._size)
+
+
 _PINNED = _PinnedPool()
 
 
@@ -346,9 +398,7 @@ def _result_array(n: int, dtype) -> np.ndarray:
     """An uninitialised array the library writes whole."""
     nbytes = n * np.dtype(dtype).itemsize
     if nbytes >= _PinnedPool.MIN:
-        raw = _PINNED.take(nbytes)
-        if raw is not None:
-            return raw[:nbytes].view(dtype)
+        return _PINNED.result(nbytes)[:nbytes].view(dtype)
     return np.empty(n, dtype=dtype)
 
 
