@@ -238,6 +238,21 @@ int handover_wait(tgp_ctx* ctx, const ResultOut& out) {
     return TGP_OK;
 }
 
+// Waits for the context's stream at the end of a scope: copies into the caller's
+// memory may be under way at every return after the first, failed or not.
+struct CopiesLanded {
+    tgp_ctx* ctx;
+    explicit CopiesLanded(tgp_ctx* c) : ctx(c) {}
+    ~CopiesLanded() {
+        if (ctx) cudaStreamSynchronize(ctx->stream);
+    }
+    cudaError_t wait() {   // the wait of the successful return
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        ctx = nullptr;
+        return e;
+    }
+};
+
 // Copies `bytes` from device memory to `dst` (host or device).
 int copy_out(tgp_ctx* ctx, void* dst, const void* src_dev, size_t bytes) {
     if (bytes == 0) return TGP_OK;
@@ -1776,19 +1791,14 @@ static int filter_impl(tgp_ctx* ctx, const Table* T, const tgp_pred_node* pred, 
         return TGP_OK;
     }
     if (rowids && ntiles && cnt) TGP_CUDA(tile_prefix(tc, tb, ntiles, cub_tmp, &cub_bytes, ctx->stream));
+    CopiesLanded copies(ctx);
     if (bitmap_out) TGP_TRY(copy_out(ctx, bitmap_out, bm, (T->rows + 7) / 8));
     if (rowids) {
-        if (!alloc && cnt > rowids_cap) {
-            TGP_CUDA(cudaStreamSynchronize(ctx->stream));
-            return fail(ctx, TGP_CAPACITY, "row-id buffer too small");
-        }
+        if (!alloc && cnt > rowids_cap) return fail(ctx, TGP_CAPACITY, "row-id buffer too small");
         if (ntiles && cnt) {
             if (alloc) {
                 rowids_out = static_cast<uint32_t*>(alloc(user, cnt));
-                if (!rowids_out) {
-                    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
-                    return fail(ctx, TGP_OOM, "row-id buffer allocation failed");
-                }
+                if (!rowids_out) return fail(ctx, TGP_OOM, "row-id buffer allocation failed");
             }
             uint32_t* dst = rowids_out;
             uint8_t* tmp = nullptr;
@@ -1802,7 +1812,7 @@ static int filter_impl(tgp_ctx* ctx, const Table* T, const tgp_pred_node* pred, 
             if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("row ids: ") + cudaGetErrorString(e));
         }
     }
-    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
+    TGP_CUDA(copies.wait());
     return TGP_OK;
 }
 
@@ -4549,6 +4559,7 @@ static int join_pairs_impl(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_ta
     }
     if (!probe_rows || !build_rows) return fail(ctx, TGP_INVALID_ARG, "null pair buffers");
     const bool dev_out = is_device_ptr(probe_rows) && is_device_ptr(build_rows);
+    CopiesLanded copies(ctx);
     if (static_cast<uint32_t>(hb[6]) <= kPairSortMax) {
         uint8_t* buf = nullptr;   // the counts stay in the arena while the pairs are written
         if (!dev_out) TGP_TRY(dev_alloc(ctx, reinterpret_cast<void**>(&buf), n * 8, "join pairs allocation failed"));
@@ -4561,7 +4572,7 @@ static int join_pairs_impl(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_ta
             if (e == cudaSuccess && !one) e = cudaMemcpyAsync(build_rows, sb, n * 4, cudaMemcpyDefault, ctx->stream);
             dev_free(ctx, buf);
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e == cudaSuccess) e = copies.wait();
         if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("join pairs: ") + cudaGetErrorString(e));
         return TGP_OK;
     }
@@ -4599,7 +4610,7 @@ static int join_pairs_impl(tgp_ctx* ctx, tgp_join_id join, tgp_table_id probe_ta
     }
     uint32_t err = 0;
     TGP_CUDA(cudaMemcpyAsync(&err, P.err, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    TGP_CUDA(cudaStreamSynchronize(ctx->stream));
+    TGP_CUDA(copies.wait());
     return check_kernel_err(ctx, err);
 }
 
