@@ -1,6 +1,9 @@
 """When a large result gets a page-locked buffer, on the CPU with the locking
 counted: never for results that are kept or larger than the pool keeps idle,
 once for results that are dropped, whatever else lies idle."""
+import gc
+import threading
+
 import numpy as np
 import pytest
 
@@ -79,3 +82,40 @@ def test_idle_buffers_make_room_below_the_limit(pool):
 def test_buffers_waste_at_most_a_quarter(pool, nbytes):
     size = pool._size(nbytes)
     assert nbytes <= size <= nbytes * 1.25 and pool._size(size) == size
+
+
+def test_arrays_dropped_by_a_collection_at_any_point(pool):
+    """Arrays in reference cycles come back while take() runs, on every thread:
+    no buffer is lost, none is handed out twice."""
+    class Node:
+        def __init__(self, a):
+            self.a, self.me = a, self
+
+    stop, bad = threading.Event(), []
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        while not stop.is_set():
+            a = pool.take(int(rng.integers(1, 9)) * MB)
+            if a is None:
+                gc.collect()
+                continue
+            a[:8] = seed
+            Node(a)
+            if not (a[:8] == seed).all():
+                bad.append(seed)
+    old = gc.get_threshold()
+    gc.set_threshold(5)
+    try:
+        ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+        [t.start() for t in ts]
+        stop.wait(3)
+        stop.set()
+        [t.join() for t in ts]
+    finally:
+        gc.set_threshold(*old)
+    gc.collect()
+    idle = [b for free in pool._idle.values() for b in free]
+    assert not bad and not pool._returned
+    assert pool._bytes == pool._idle_bytes == sum(b.nbytes for b in idle) <= pool.KEEP
+    assert sorted(pool.locked) == sorted(pool.unlocked + [b.nbytes for b in idle])

@@ -10,6 +10,7 @@ back to the CPU.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import sys
 import threading
@@ -278,16 +279,18 @@ class _PinnedPool:
 
     An array holds its buffer until it and every view of it are gone; then the
     buffer serves the next result. All buffers together stay within LIMIT bytes
-    and the idle ones within KEEP (the ones idle longest are unlocked and
-    freed); past LIMIT, or without a device, results are ordinary arrays."""
+    and the idle ones within KEEP (those of the size left alone longest are
+    unlocked and freed); past LIMIT, or without a device, results are ordinary
+    arrays."""
 
     MIN = 1 << 20
     KEEP = 256 << 20
     LIMIT = 1 << 30
 
     def __init__(self):
-        self._lock = threading.RLock()   # re-entered when a collection inside a call drops an array
-        self._idle: list[np.ndarray] = []   # longest idle first
+        self._lock = threading.Lock()   # holders settle what came back meanwhile
+        self._returned: collections.deque = collections.deque()   # buffers whose arrays are gone, not yet idle
+        self._idle: dict[int, list] = {}   # by size, the size returned to last at the end; no empty list
         self._idle_bytes = self._bytes = 0
         self._dropped: set[int] = set()   # buffer sizes of which an ordinary array was dropped
 
@@ -300,38 +303,42 @@ class _PinnedPool:
     def result(self, nbytes: int) -> np.ndarray:
         """A uint8 array of at least nbytes for one result."""
         size = self._size(nbytes)
-        with self._lock:
-            locked = size <= self.KEEP and (size in self._dropped or any(b.nbytes == size for b in self._idle))
-            if locked and not any(b.nbytes == size for b in self._idle):
-                self._dropped.discard(size)
-        raw = self.take(nbytes) if locked else None
+        raw = None
+        if size in self._idle or size in self._dropped:
+            raw = self._take(size)
         return np.asarray(_OrdinaryLease(self, np.empty(nbytes, dtype=np.uint8), size)) if raw is None else raw
 
     def take(self, nbytes: int) -> np.ndarray | None:
         """A page-locked uint8 array of at least nbytes, or None."""
-        size = self._size(nbytes)
+        return self._take(self._size(nbytes))
+
+    def _take(self, size: int) -> np.ndarray | None:
+        buf, room, fits = None, [], False
         with self._lock:
-            for i in range(len(self._idle) - 1, -1, -1):
-                if self._idle[i].nbytes == size:
-                    buf = self._idle.pop(i)
-                    self._idle_bytes -= size
-                    return np.asarray(_PinnedLease(self, buf))
-            room = self._trim(self.KEEP, self.LIMIT - size)
-            fits = self._bytes + size <= self.LIMIT
-            if fits:
-                self._bytes += size
-        self._free(room)
-        if not fits:
-            return None
-        buf = None
-        try:
-            buf = self._register(size)
-        except Exception:   # no memory, no library: an ordinary array serves
-            pass
-        finally:
-            if buf is None:
-                with self._lock:
-                    self._bytes -= size
+            free = self._idle.get(size)
+            if free:
+                buf = free.pop()
+                if not free:
+                    del self._idle[size]
+                self._idle_bytes -= size
+            else:
+                self._dropped.discard(size)
+                room = self._trim(self.LIMIT - size)
+                fits = self._bytes + size <= self.LIMIT
+                if fits:
+                    self._bytes += size
+        if room or self._returned:
+            self._settle(room)
+        if fits:
+            try:
+                buf = self._register(size)
+            except Exception:   # no memory, no library: an ordinary array serves
+                pass
+            finally:
+                if buf is None:
+                    with self._lock:
+                        self._bytes -= size
+                    self._settle([])
         return None if buf is None else np.asarray(_PinnedLease(self, buf))
 
     @staticmethod
@@ -343,26 +350,42 @@ class _PinnedPool:
     def _unregister(buf: np.ndarray) -> None:
         A.load().tgp_host_unlock(buf.ctypes.data)
 
-    def _trim(self, idle: int, total: int) -> list:
-        """Takes the longest idle buffers out until the bounds hold, or none is idle."""
+    def _trim(self, total: int) -> list:
+        """Takes idle buffers out until the bounds hold, or none is idle (the lock is held)."""
         out = []
-        while self._idle and (self._idle_bytes > idle or self._bytes > total):
-            buf = self._idle.pop(0)
-            self._idle_bytes -= buf.nbytes
-            self._bytes -= buf.nbytes
-            out.append(buf)
+        while self._idle and (self._idle_bytes > self.KEEP or self._bytes > total):
+            size = next(iter(self._idle))
+            out.append(self._idle[size].pop(0))
+            if not self._idle[size]:
+                del self._idle[size]
+            self._idle_bytes -= size
+            self._bytes -= size
         return out
 
-    def _free(self, bufs: list) -> None:
-        for buf in bufs:
-            self._unregister(buf)
-
     def _give(self, buf: np.ndarray) -> None:
-        with self._lock:
-            self._idle.append(buf)
-            self._idle_bytes += buf.nbytes
-            out = self._trim(self.KEEP, self.LIMIT)
-        self._free(out)
+        # An array can be dropped at any point, by a collection inside take()
+        # too: the buffer is queued, and whoever gets the lock sorts it in.
+        self._returned.append(buf)
+        self._settle([])
+
+    def _settle(self, out: list) -> None:
+        """Unlocks `out`, then makes the returned buffers idle. A holder of the
+        lock does this after releasing it, so no buffer waits for the next call."""
+        while True:
+            for buf in out:
+                self._unregister(buf)
+            if not self._returned or not self._lock.acquire(blocking=False):
+                return
+            try:
+                while self._returned:
+                    buf = self._returned.popleft()
+                    size = buf.nbytes
+                    self._idle.setdefault(size, []).append(buf)
+                    self._idle[size] = self._idle.pop(size)
+                    self._idle_bytes += size
+                out = self._trim(self.LIMIT)
+            finally:
+                self._lock.release()
 
 
 class _PinnedLease:
