@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "batch_lanes.hpp"
+#include "cpu_relax.hpp"
 #include "runtime.hpp"
 
 using namespace tgp;
@@ -225,7 +226,7 @@ int handover_wait(tgp_ctx* ctx, const ResultOut& out) {
     const volatile unsigned long long* flag = ctx->rhost + 2ull * out.words16;
     const auto t0 = std::chrono::steady_clock::now();
     for (uint32_t i = 1; *flag != out.seq; ++i) {
-        __builtin_ia32_pause();
+        cpu_relax();
         if ((i & 255u) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
             const cudaError_t e = cudaStreamSynchronize(ctx->stream);
             if (e != cudaSuccess || *flag != out.seq)
