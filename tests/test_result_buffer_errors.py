@@ -26,6 +26,19 @@ def test_a_failed_lock_gives_an_ordinary_array(monkeypatch, error):
     assert pool._bytes == pool._idle_bytes == 0
 
 
+@pytest.mark.parametrize("error", [MemoryError, KeyboardInterrupt])
+def test_an_error_while_the_result_is_allocated_is_raised_as_itself(monkeypatch, error):
+    def no_array(n, dtype):
+        raise error("no room")
+
+    def call(alloc):
+        if alloc(None, 5) is None:
+            raise engine.A.TgpError(engine.A.OOM, "row-id buffer allocation failed")
+    monkeypatch.setattr(engine, "_result_array", no_array)
+    with pytest.raises(error, match="no room"):
+        engine._result_words(call)
+
+
 PROGRAM = """
 import sys
 sys.modules["torch"] = None      # not installed

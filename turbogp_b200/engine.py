@@ -428,16 +428,21 @@ def _result_array(n: int, dtype) -> np.ndarray:
 def _result_words(call) -> np.ndarray:
     """The u32 result of call(alloc), allocated by the library (tgp_alloc_fn)
     once its length is known; empty when it allocates nothing."""
-    got = []
+    got, failed = [], []
 
     def alloc(_user, count):
         try:
             got.append(_result_array(int(count), np.uint32))
-        except Exception:   # the library reports the failed allocation
+        except BaseException as e:   # cannot pass through the library: raised after it
+            failed.append(e)
             return None
         return got[-1].ctypes.data
 
-    call(A.AllocFn(alloc))
+    try:
+        call(A.AllocFn(alloc))
+    finally:
+        if failed:
+            raise failed[0]
     return got[-1] if got else np.empty(0, dtype=np.uint32)
 
 
