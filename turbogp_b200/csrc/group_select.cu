@@ -445,8 +445,7 @@ cudaError_t top_select_narrow(const unsigned long long* htab, uint64_t max_group
     top_bucket_kernel<<<1, 1024, 0, st>>>(hist, state);
     top_split_kernel<<<grid, kTopThreads, 0, st>>>(in, next, sure, state);
     const size_t smem = kTopSort * sizeof(TopCand);
-    cudaError_t e = cudaFuncSetAttribute(top_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(&top_finish_kernel), smem);
     if (e != cudaSuccess) return e;
     top_finish_kernel<<<1, 1024, smem, st>>>(htab, next, sure, state, F, limit, keys_out, vals_out);
     return cudaGetLastError();

@@ -376,7 +376,7 @@ uint64_t group_stream_rows_per_cta(uint64_t nrows, int sms) {
 
 cudaError_t launch_group_stream(const GroupStreamArgs& A, int vs, int pay, uint32_t smem, int grid, cudaStream_t st) {
     const void* f = vs == GS_COLS ? gs_kernel<GS_COLS>(pay) : vs == GS_Q1 ? gs_kernel<GS_Q1>(pay) : gs_kernel<GS_JOIN>(pay);
-    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = allow_dynamic_smem(f, smem);
     if (e != cudaSuccess) return e;
     GroupStreamArgs a = A;
     void* args[] = {&a};

@@ -664,9 +664,7 @@ int direct_group_ctas_per_sm(uint32_t hs, bool hasv) {
     const void* f = dg_kernel(DT_I64, hasv ? DT_I32 : 0);
     int occ = 0;
     const size_t smem = static_cast<size_t>(hs) * (hasv ? 12 : 8);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-        return 0;
+    if (allow_dynamic_smem(f, smem) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, kDgThreads, smem) != cudaSuccess) return 0;
     return occ;
 }
@@ -680,9 +678,7 @@ cudaError_t launch_hash_group(const HashGroupArgs& A, uint32_t kdt, uint32_t vdt
     a.hs = A.hs ? kHgSlots : 0u;
     a.hs_log2 = a.hs ? 31u - static_cast<uint32_t>(__builtin_clz(a.hs)) : 0u;
     const size_t smem = static_cast<size_t>(a.hs) * 16 + (kDgThreads / 32) * kHgQueue * (a.hs ? 16 : 20);
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024)
-        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = allow_dynamic_smem(f, smem);
     if (e != cudaSuccess) return e;
     void* args[] = {&a};
     return cudaLaunchKernel(f, dim3(static_cast<unsigned>(hash_group_grid(A.nrows, sms))), dim3(kDgThreads), args, smem, st);
@@ -706,9 +702,7 @@ size_t q1_group_smem(uint32_t ngroups) { return static_cast<size_t>(ngroups) * k
 int q1_group_ctas_per_sm(uint32_t ngroups) {
     const void* f = reinterpret_cast<const void*>(&q1_group_kernel);
     const size_t smem = q1_group_smem(ngroups);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-        return 0;
+    if (allow_dynamic_smem(f, smem) != cudaSuccess) return 0;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, kDgThreads, smem) != cudaSuccess) return 0;
     return occ;
@@ -717,10 +711,8 @@ int q1_group_ctas_per_sm(uint32_t ngroups) {
 cudaError_t launch_q1_group(const Q1Args& A, int grid, cudaStream_t st) {
     const void* f = reinterpret_cast<const void*>(&q1_group_kernel);
     const size_t smem = q1_group_smem(A.ngroups);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_dynamic_smem(f, smem);
+    if (e != cudaSuccess) return e;
     Q1Args a = A;
     void* args[] = {&a};
     return cudaLaunchKernel(f, dim3(static_cast<unsigned>(grid)), dim3(kDgThreads), args, smem, st);
@@ -730,10 +722,8 @@ cudaError_t launch_direct_group(const DirectGroupArgs& A, uint32_t kdt, uint32_t
     const void* f = dg_kernel(kdt, vdt);
     if (!f) return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(A.hs) * (vdt ? 12 : 8);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_dynamic_smem(f, smem);
+    if (e != cudaSuccess) return e;
     DirectGroupArgs a = A;
     void* args[] = {&a};
     return cudaLaunchKernel(f, dim3(static_cast<unsigned>(grid)), dim3(kDgThreads), args, smem, st);

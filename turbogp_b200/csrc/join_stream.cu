@@ -214,7 +214,7 @@ cudaError_t launch_join_stream(const JoinStreamArgs& A, bool bits, int grid, cud
     const void* f = bits ? reinterpret_cast<const void*>(&join_stream_kernel<true>)
                          : reinterpret_cast<const void*>(&join_stream_kernel<false>);
     const size_t smem = join_stream_smem(A.table_bytes, A.copies, A.ngroups);
-    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = allow_dynamic_smem(f, smem);
     if (e != cudaSuccess) return e;
     JoinStreamArgs a = A;
     void* args[] = {&a};

@@ -65,6 +65,10 @@ struct Q1Args {
     unsigned long long* counters;
     ResultOut out;
 };
+// Lets kernel `f` have `bytes` of dynamic shared memory. The limit belongs to the
+// process and only ever rises: another thread's smaller launch of the same
+// kernel cannot lower it between this call and the launch it is for.
+cudaError_t allow_dynamic_smem(const void* f, size_t bytes);
 // GROUP BY one sparse key into 16-byte hash slots [key][count << shift + sum]
 // under at most four int32 leaves (groupby_direct.cu). hs: keep the per-CTA
 // shared table (no CTA's i32 partial can reach 2^31 over

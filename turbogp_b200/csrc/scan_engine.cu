@@ -2613,7 +2613,7 @@ struct KernelCacheEntry {
 };
 
 static std::mutex g_kcache_mu;
-static KernelCacheEntry g_kcache[128];
+static KernelCacheEntry g_kcache[1024];   // kernels x devices
 static int g_kcache_n = 0;
 
 static KernelCacheEntry* kernel_entry(const void* f) {
@@ -2635,6 +2635,11 @@ static cudaError_t ensure_smem_limit(KernelCacheEntry* e, const void* f, int sme
     const cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (r == cudaSuccess && e) e->smem_limit = smem;
     return r;
+}
+
+cudaError_t allow_dynamic_smem(const void* f, size_t bytes) {
+    std::lock_guard<std::mutex> lock(g_kcache_mu);
+    return ensure_smem_limit(kernel_entry(f), f, static_cast<int>(bytes));
 }
 
 // Launches with blockDim = nthreads consumers + one producer warp.
