@@ -698,8 +698,8 @@ typedef struct tgp_tune_entry {
                                queued behind a short device delay) */
     int32_t status;         /* TGP_OK, or why the candidate could not run */
     uint32_t same_result;   /* 1 = its result equals the planner's rule's, bit for bit */
-    uint32_t threads_used;  /* what the plan launched with */
-    uint32_t stages_used;
+    uint32_t threads_used;  /* threads per CTA (without the producer warp) and shared-memory stages of the */
+    uint32_t stages_used;   /* launch; 0 stages: a streaming kernel, which reads rows straight from memory */
     uint32_t mode_used;     /* accumulator placement the plan chose: 2 private, 3 shared, 4 global, 5 hash,
                                8 per-warp 32-bit limb tables */
     uint32_t _pad;

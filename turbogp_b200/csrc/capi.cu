@@ -859,6 +859,11 @@ int size_planned(tgp_ctx* ctx, Plan& P, uint32_t mode, bool acc128, size_t extra
     return size_smem(ctx, P, extra, stat, &kn);
 }
 
+void launched(tgp_ctx* ctx, uint32_t threads, uint32_t stages) {
+    ctx->launched_threads = threads;
+    ctx->launched_stages = stages;
+}
+
 // With profiling on, takes the next pair of timing events and records the
 // first on the context's stream (after a bounded device delay when gated);
 // *ev stays null otherwise.
@@ -901,6 +906,7 @@ int launch(tgp_ctx* ctx, const Plan& P0, uint32_t mode, bool acc128) {
     TGP_TRY(profile_begin(ctx, &ev));
     cudaError_t e = launch_scan(P, mode, acc128, static_cast<int>(grid), ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("scan launch: ") + cudaGetErrorString(e));
+    launched(ctx, P.nthreads, P.nstages);
     if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
     return TGP_OK;
 }
@@ -951,6 +957,7 @@ int launch_direct_groups(tgp_ctx* ctx, const Plan& P, uint64_t max_abs_val) {
     TGP_TRY(profile_begin(ctx, &ev));
     cudaError_t e = launch_direct_group(A, kdt, vdt, static_cast<int>(grid), ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("group launch: ") + cudaGetErrorString(e));
+    launched(ctx, kDirectThreads, 0);
     if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
     return TGP_OK;
 }
@@ -993,6 +1000,7 @@ int launch_hash_groups(tgp_ctx* ctx, const Plan& P, uint64_t max_abs_val) {
     TGP_TRY(profile_begin(ctx, &ev));
     const cudaError_t e = launch_hash_group(A, kdt, vdt, ctx->sms, ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("group launch: ") + cudaGetErrorString(e));
+    launched(ctx, kDirectThreads, 0);
     if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
     return TGP_OK;
 }
@@ -1061,6 +1069,7 @@ int try_launch_q1(tgp_ctx* ctx, const Plan& P, uint32_t mode, bool acc128, uint6
     TGP_TRY(profile_begin(ctx, &ev));
     const cudaError_t e = launch_q1_group(A, static_cast<int>(grid), ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("grouped launch: ") + cudaGetErrorString(e));
+    launched(ctx, kDirectThreads, 0);
     if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
     *done = true;
     return TGP_OK;
@@ -1123,6 +1132,7 @@ int try_launch_join(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroups
     TGP_TRY(profile_begin(ctx, &ev));
     const cudaError_t e = launch_join_stream(A, look.bits, static_cast<int>(grid), ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("join launch: ") + cudaGetErrorString(e));
+    launched(ctx, kStreamThreads, 0);
     if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
     *done = true;
     return TGP_OK;
@@ -1268,6 +1278,7 @@ int try_launch_group(tgp_ctx* ctx, const Plan& P, uint32_t mode, uint64_t ngroup
     const cudaError_t e = launch_group_stream(A, vs, pay, static_cast<uint32_t>(off + A.copies * entry), static_cast<int>(grid),
                                               ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TGP_DEVICE_ERROR, std::string("group launch: ") + cudaGetErrorString(e));
+    launched(ctx, kStreamThreads, 0);
     if (ev) TGP_CUDA(cudaEventRecord(ev->second, ctx->stream));
     *done = true;
     return TGP_OK;
@@ -3310,13 +3321,13 @@ int tgp_autotune(tgp_ctx* ctx, const tgp_query* q, uint32_t reps, tgp_tune_entry
         QueryState qs;
         e.status = plan_query(ctx, q, qs, scan_kernel_static_smem(), nullptr, /*dry=*/true);
         if (e.status == TGP_OK) {
-            e.threads_used = qs.mode == MODE_GROUP_PRIVATE ? qs.b->P.nthreads : 512u;
             e.mode_used = qs.mode;
-            Plan P = qs.b->P;
-            if (size_smem(ctx, P, qs.extra, scan_kernel_static_smem(), &qs.kn) == TGP_OK) e.stages_used = P.nstages;
             HostResult r;
             r.res.ngroups = ref.res.ngroups;
+            launched(ctx, 0, 0);
             e.status = run_into(ctx, q, &r);
+            e.threads_used = ctx->launched_threads;
+            e.stages_used = ctx->launched_stages;
             e.same_result = (e.status == TGP_OK && same_results(q, ref, r)) ? 1u : 0u;
         }
         if (e.status == TGP_OK && e.same_result) {

@@ -28,7 +28,7 @@ namespace tgp {
 
 namespace {
 
-constexpr int kGsThreads = 1024;
+constexpr int kGsThreads = kStreamThreads;
 constexpr int kGsWarps = kGsThreads / 32;
 constexpr int kGsRows = 128;
 constexpr uint32_t kGsNone = 0xffu;   // payload byte: no match

@@ -28,7 +28,7 @@ namespace tgp {
 
 namespace {
 
-constexpr int kDgThreads = 512;
+constexpr int kDgThreads = kDirectThreads;
 // Two CTAs per SM (64 registers, no spills) with two warp chunks' loads in
 // flight measured faster on B200 (20M rows, 10M key range, Zipf(1.1)) than
 // three CTAs with one or two chunks (40 registers) and two CTAs with three.

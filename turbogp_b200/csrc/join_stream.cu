@@ -36,7 +36,7 @@ namespace tgp {
 
 namespace {
 
-constexpr int kJsThreads = 1024;
+constexpr int kJsThreads = kStreamThreads;
 constexpr int kJsWarps = kJsThreads / 32;
 constexpr int kJsRows = 128;   // rows per warp chunk, four consecutive per lane
 

@@ -65,6 +65,9 @@ struct Q1Args {
     unsigned long long* counters;
     ResultOut out;
 };
+// Threads per CTA of the direct-group, hash-group and Q1 kernels, and of the
+// streaming joins and limb tables.
+constexpr int kDirectThreads = 512, kStreamThreads = 1024;
 // Lets kernel `f` have `bytes` of dynamic shared memory. The limit belongs to the
 // process and only ever rises: another thread's smaller launch of the same
 // kernel cannot lower it between this call and the launch it is for.
@@ -432,6 +435,9 @@ struct tgp_ctx {
     unsigned long long* rblock = nullptr;
     unsigned long long* rhost = nullptr;
     uint32_t rseq = 0;
+    // The last scan launch's threads per CTA and shared-memory stages (0: the
+    // kernel has none), for the autotuner's report.
+    uint32_t launched_threads = 0, launched_stages = 0;
     bool rdirty = false;   // not handed over since its last use: clear the block first
     // Device staging of kernel-table inputs (kept apart from the arena so
     // scans that grow the arena never move a staged input).
