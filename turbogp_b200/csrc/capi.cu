@@ -2275,7 +2275,9 @@ static int plan_query(tgp_ctx* ctx, const tgp_query* q, QueryState& qs, size_t s
             }
             // Dense column program: int64 partials, no join, no per-row
             // overflow checks.
-            if (!acc128 && (!J || pay_ok) && !P.check_ovf && kn.dense && !bucket)
+            // It adds a thread's rows of a tile between two checks of the flush
+            // limit, so the limit has to be above them (for values below 2^59 it is).
+            if (!acc128 && (!J || pay_ok) && !P.check_ovf && kn.dense && !bucket && P.flush_limit > kTileRows / nt)
                 P.dense_vec = compile_chain(b, pay_ok) ? 1u : 0u;
             // Scalar aggregates prefer the register fast path; a join's dense
             // program implies its payload path.

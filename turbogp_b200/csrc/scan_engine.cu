@@ -1095,9 +1095,10 @@ __device__ __forceinline__ void chain_private_tile(const Plan& P, uint8_t* extra
     constexpr int R = kTileRows / NT;
     unsigned long long* w = reinterpret_cast<unsigned long long*>(extra);
     // The int64 partials stay below 2^63 in magnitude: flush before this
-    // tile's updates could pass the host's bound.
+    // tile's updates could reach the host's bound (which is above a tile's, so
+    // the row paths find room for the update that they add before they check).
     const uint32_t nsel = __popc(m);
-    if (sink.upd + nsel > P.flush_limit) {
+    if (sink.upd + nsel >= P.flush_limit) {
         sink.flush_private_thread(P, extra, t);
         sink.upd = 0;
     }
@@ -1445,7 +1446,7 @@ __device__ __forceinline__ void chain_tile_static(const Plan& P, uint8_t* extra,
     });
 
     const uint32_t nsel = __popc(m);
-    if (sink.upd + nsel > P.flush_limit) {
+    if (sink.upd + nsel >= P.flush_limit) {
         sink.flush_private_thread(P, extra, t);
         sink.upd = 0;
     }
