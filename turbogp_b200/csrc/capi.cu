@@ -4338,6 +4338,7 @@ int tgp_graph_capture(tgp_ctx* ctx, const tgp_query* q, tgp_graph_id* out) {
         TGP_TRY(upload(ctx, g.image, img.data(), img.size() * 8));
     }
     TGP_TRY(size_planned(ctx, P, qs.mode, qs.acc128, qs.extra, qs.kn));
+    bound_presum(ctx, qs);
     // Kernel attributes and occupancy are settled before the capture.
     if (scan_occupancy(qs.mode, qs.acc128, static_cast<int>(P.nthreads), P.smem_bytes, P.shape, P.two_ctas != 0) <= 0)
         return fail(ctx, TGP_DEVICE_ERROR, "scan kernel cannot be resident with this shared memory");
