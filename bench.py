@@ -975,6 +975,9 @@ def run_headline(args, world: int, rank: int, local: int) -> None:
     query = table.prepare(tpl.aggs, tpl.group_by, tpl.where)
     first = query.run()
     tune = None if args.no_autotune else autotune_summary(ctx, query)
+    # Threads per CTA of the scan: the tuned variant's, else the rule's (two
+    # CTAs of 256 from four tiles per CTA on).
+    scan_threads = tune["chosen_threads"] if tune else 256 if rows >= 8 * ctx.sm_count * 2048 else 512
     # Warm-up.
     for _ in range(args.warmup):
         out = query.run()
@@ -1067,7 +1070,7 @@ def run_headline(args, world: int, rank: int, local: int) -> None:
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic_per_launch(),
                      "kernel_ms": kernel_avg_ms, "kernel_ms_ungated": kernel_avg_ungated_ms,
                      "timing": "device events around each launch, launch queued behind a device delay",
-                     "kernel": "scan_kernel<MODE_GROUP_PRIVATE, int64, 512, ScalarTag>"},
+                     "kernel": f"scan_kernel<MODE_GROUP_PRIVATE, int64, {scan_threads}, ScalarTag>"},
         "e2e": {"value": e2e_value, "unit": "rows/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "cpu_baseline": cpu,
         "clocks": clk,
