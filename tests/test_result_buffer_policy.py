@@ -84,6 +84,28 @@ def test_buffers_waste_at_most_a_quarter(pool, nbytes):
     assert nbytes <= size <= nbytes * 1.25 and pool._size(size) == size
 
 
+def test_release_gives_the_idle_buffers_back(pool):
+    held = pool.take(4 * MB)
+    for _ in range(3):
+        array(12 * MB)
+    pool.take(2 * MB)
+    assert pool._idle_bytes == 14 * MB
+    pool.release()
+    assert sorted(pool.unlocked) == [2 * MB, 12 * MB] and pool._idle_bytes == 0 and pool._bytes == 4 * MB
+    del held
+    assert pool._bytes == pool._idle_bytes == 4 * MB      # on loan meanwhile: idle now
+
+
+@pytest.mark.gpu
+def test_a_closed_context_keeps_no_idle_buffer():
+    with engine.Context(0) as ctx:
+        t = ctx.register({"k": np.zeros(4_000_000, dtype=np.int32)}, {"k": "int"})
+        for _ in range(4):
+            assert t.filter(engine.col("k") < 1).count == 4_000_000
+        assert engine._PINNED._idle_bytes >= 16_000_000
+    assert engine._PINNED._idle_bytes == 0
+
+
 def test_arrays_dropped_by_a_collection_at_any_point(pool):
     """Arrays in reference cycles come back while take() runs, on every thread:
     no buffer is lost, none is handed out twice."""

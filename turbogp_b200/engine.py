@@ -280,8 +280,8 @@ class _PinnedPool:
     An array holds its buffer until it and every view of it are gone; then the
     buffer serves the next result. All buffers together stay within LIMIT bytes
     and the idle ones within KEEP (those of the size left alone longest are
-    unlocked and freed); past LIMIT, or without a device, results are ordinary
-    arrays."""
+    unlocked and freed), and a context that closes gives the idle ones back; past
+    LIMIT, or without a device, results are ordinary arrays."""
 
     MIN = 1 << 20
     KEEP = 256 << 20
@@ -361,6 +361,15 @@ class _PinnedPool:
             self._idle_bytes -= size
             self._bytes -= size
         return out
+
+    def release(self) -> None:
+        """Unlocks and frees the idle buffers."""
+        with self._lock:
+            out = [buf for free in self._idle.values() for buf in free]
+            self._idle.clear()
+            self._idle_bytes -= sum(buf.nbytes for buf in out)
+            self._bytes -= sum(buf.nbytes for buf in out)
+        self._settle(out)
 
     def _give(self, buf: np.ndarray) -> None:
         # An array can be dropped at any point, by a collection inside take()
@@ -465,6 +474,7 @@ class Context:
         if getattr(self, "h", None):
             self.lib.tgp_shutdown(self.h)
             self.h = None
+            _PINNED.release()
 
     def __enter__(self):
         return self
@@ -990,7 +1000,8 @@ class PreparedQuery:
         """Records the query as a CUDA graph (tgp_graph_capture); later ``run``
         calls replay it with one graph launch and no planning. Direct-indexed
         and scalar aggregates only (a hash-grouped query raises TgpError
-        UNSUPPORTED)."""
+        UNSUPPORTED). A replay runs the scan pipeline's kernels, also where an
+        uncaptured ``run`` has a faster streaming kernel."""
         ctx = self.table.ctx
         self.drop_graph()
         gid = C.c_uint64()
