@@ -373,26 +373,42 @@ class _PinnedPool:
 
     def _give(self, buf: np.ndarray) -> None:
         # An array can be dropped at any point, by a collection inside take()
-        # too: the buffer is queued, and whoever gets the lock sorts it in.
-        self._returned.append(buf)
-        self._settle([])
+        # too: a buffer that finds the lock taken is queued, and whoever holds it
+        # sorts it in.
+        if not self._lock.acquire(False):
+            self._returned.append(buf)
+            return self._settle([])
+        try:
+            out = self._shelve(buf)
+        finally:
+            self._lock.release()
+        if out or self._returned:
+            self._settle(out)
+
+    def _shelve(self, buf: np.ndarray) -> list:
+        """Makes a buffer idle; the ones that no longer fit (the lock is held)."""
+        size = buf.nbytes
+        free = self._idle.pop(size, None)
+        if free is None:
+            self._idle[size] = [buf]
+        else:
+            free.append(buf)
+            self._idle[size] = free
+        self._idle_bytes += size
+        return self._trim(self.LIMIT) if self._idle_bytes > self.KEEP or self._bytes > self.LIMIT else []
 
     def _settle(self, out: list) -> None:
-        """Unlocks `out`, then makes the returned buffers idle. A holder of the
+        """Unlocks `out`, then makes the queued buffers idle. A holder of the
         lock does this after releasing it, so no buffer waits for the next call."""
         while True:
             for buf in out:
                 self._unregister(buf)
-            if not self._returned or not self._lock.acquire(blocking=False):
+            if not self._returned or not self._lock.acquire(False):
                 return
+            out = []
             try:
                 while self._returned:
-                    buf = self._returned.popleft()
-                    size = buf.nbytes
-                    self._idle.setdefault(size, []).append(buf)
-                    self._idle[size] = self._idle.pop(size)
-                    self._idle_bytes += size
-                out = self._trim(self.LIMIT)
+                    out += self._shelve(self._returned.popleft())
             finally:
                 self._lock.release()
 
