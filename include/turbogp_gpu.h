@@ -593,6 +593,10 @@ TGP_API int tgp_batch_poll(tgp_ctx* ctx, tgp_batch_id batch, int wait);
  * proven from them); otherwise the launch returns TGP_NOT_FOUND as well. */
 typedef uint64_t tgp_graph_id;
 
+/* A captured query runs the scan pipeline's kernels. tgp_execute has streaming
+ * kernels for some shapes (grouping by two flags with the TPC-H Q1 values, groups
+ * of up to a few thousand, joins on unique keys) and hands small results over
+ * without a copy: for those it is the faster way, replay saves the planning only. */
 TGP_API int tgp_graph_capture(tgp_ctx* ctx, const tgp_query* q, tgp_graph_id* out);
 
 /* Runs a captured query on the context's stream and waits for it; outputs as

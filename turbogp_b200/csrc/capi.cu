@@ -27,7 +27,12 @@ namespace {
 constexpr unsigned long long kEmptySlot = ~0ull;
 constexpr uint64_t kDirectMaxGroups = 1ull << 22;
 constexpr uint64_t kHashDirectMax = 1ull << 27;   // key values of a directly indexed group table
-constexpr uint64_t kDeviceFormatGroups = 4096;         // direct groups formatted on the device from here on
+// Direct groups formatted on the device from here on: one wait either way, but a
+// kernel more against a host thread's decoding. Queries of 1 / 2 / 5 aggregates,
+// host against device: 2,048 groups 40 / 49 / 87 us against 47 / 62 / 98, 3,000
+// groups 47 / 58 / 104 against 50 / 65 / 111, 4,000 groups 54 / 70 / 134 against
+// 52 / 70 / 122.
+constexpr uint64_t kDeviceFormatGroups = 4096;
 constexpr size_t kOnePassBytes = 1536u << 10;          // results formatted with room for every slot (30 us of link)
 constexpr size_t kStagedResultBytes = 4u << 20;        // formatted results that come back through ctx->hpin
 // Join payloads the streaming probe keeps in a CTA's shared memory: the bytes
@@ -833,11 +838,12 @@ int size_smem(tgp_ctx* ctx, Plan& P, size_t extra_bytes, size_t static_smem = sc
 // Shared-memory stages of a planned query. Scalar aggregates over many tiles
 // (register fast path) run as two CTAs of 256 threads per SM, each with half
 // the stage ring, instead of one of 512: while one CTA's consumers wait for a
-// stage the other's run. 60M rows of 20 bytes, B200: kernel 194 -> 179 us (with
-// the results handed over; 185 -> 173 without). From four tiles per CTA on
-// (2.4M rows): queries of 2.5-9M rows take 0.90-1.03 of their time with one CTA,
-// smaller ones the same within noise. A variant that names threads, stages
-// or CTAs is left as it is.
+// stage the other's run. 60M rows of 20 bytes, B200: kernel 190 -> 178 us. From
+// four tiles per CTA on (2.4M rows), kernel time against one CTA's (20-byte
+// rows / one 4-byte column / five columns): 2.5M rows 0.91 / 0.92 / 0.94, 5M
+// 1.00 / 0.88 / 0.87, 10M 0.96 / 0.85 / 0.84, 60M 0.94 / 0.75 / 0.75; smaller
+// queries take the same within noise. A variant that names threads, stages or
+// CTAs is left as it is.
 constexpr uint64_t kScalarPairTiles = 4;
 
 int size_planned(tgp_ctx* ctx, Plan& P, uint32_t mode, bool acc128, size_t extra, const Knobs& kn) {
@@ -2628,8 +2634,8 @@ static int shrink_group_table(tgp_ctx* ctx, QueryState& qs, bool* shrunk) {
 
 // Whether a run of the query formats its groups on the device straight from
 // their table: directly indexed slots, and direct accumulators of many groups
-// (few are decoded on the host from the one readback that carries the
-// counters, without the extra kernels and the second wait).
+// (fewer are decoded on the host from the block that carries the counters:
+// kDeviceFormatGroups).
 static bool formats_direct(const QueryState& qs, const tgp_query* q) {
     if (q->nagg > static_cast<uint32_t>(kMaxFormatAggs)) return false;
     if (qs.mode == MODE_GROUP_HASH) return qs.b->P.hdirect != 0;

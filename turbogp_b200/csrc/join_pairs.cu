@@ -16,9 +16,9 @@
 //      radix-sorted path of the scan engine).
 // Both passes stream the rows at full occupancy (no stage ring): a probe waits
 // on a dependent L2 access per step, so warps in flight set the pace. B200, 8M
-// probe rows (half selected) against 200K rows of 2-row keys, 3.9M pairs: count
-// and write 207 us each plus a radix sort of the pairs of 370 us in the scan
-// engine's form.
+// probe rows (half selected) against 200K keys of two rows, 3.9M pairs: count
+// 73 us and write 99 us; in the scan engine's form 207 us each and a radix sort
+// of the pairs of 370 us.
 #include <cuda_runtime.h>
 
 #include <cstdint>

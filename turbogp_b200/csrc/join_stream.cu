@@ -16,13 +16,16 @@
 // The bits stay below 190 KB: past 195 KB of shared memory the SM's L1 shrinks
 // to a size at which the streamed columns evict each other (60M rows x 1.5M
 // keys: 0.25 -> 0.45 ms). B200, Zipf(0.8) keys, half the build side kept,
-// query without the build: 60M x 1.5M 0.285 -> 0.242 ms (the matches' payload
-// bytes bound it), 60M x 20K 0.233 -> 0.161 ms (16 bytes per row at 0.92 of the
-// copy bandwidth), 8M x 1.5M 74 -> 54 us.
+// kernel: 60M x 1.5M 0.258-0.335 -> 0.211-0.278 ms over 14 payload arrays (the
+// matches' payload bytes bound it, and how fast they come depends on where in
+// memory the array lies; most arrays: 0.258 -> 0.221-0.248); query without the
+// build: 60M x 20K 0.233 -> 0.161 ms (16 bytes per row at 0.92 of the copy
+// bandwidth), 8M x 1.5M 74 -> 54 us.
 // One CTA of 1,024 threads per SM holds the table; a lane takes four
 // consecutive rows of a 128-row chunk with 16-byte loads. Groups accumulate in per-warp
 // tables of 32-bit limbs as in the scan engine (exact: the host proves every
-// sum below 2^63).
+// sum below 2^63). Distances from the smallest build key are taken in 32 bits:
+// the host sends only build ranges within int32 here.
 #include <cuda_runtime.h>
 
 #include <algorithm>
