@@ -61,7 +61,7 @@ fn main() {
             .arg(&obj));
         objects.push(obj);
     }
-    for header in ["device_common.cuh", "plan.hpp", "runtime.hpp"] {
+    for header in ["batch_lanes.hpp", "cpu_relax.hpp", "device_common.cuh", "group_format.cuh", "plan.hpp", "runtime.hpp"] {
         println!("cargo:rerun-if-changed={}", csrc.join(header).display());
     }
     println!("cargo:rerun-if-changed={}", include.join("turbogp_gpu.h").display());
